@@ -34,9 +34,9 @@
 #include <vector>
 
 #include "mhd_adjoint.cuh"
-#include "mhd_cg_sweep.cuh"
 #include "mhd_finalize_sweep.cuh"
 #include "mhd_host_util.h"
+#include "mhd_solve.h"
 #include "mhd_sweep.cuh"
 
 using namespace mhd;
@@ -89,14 +89,14 @@ struct mhd_adjoint {
     AdjScratch s{};
     StepCoeffs* coeffs = nullptr;
     DeviceStatus* status = nullptr;
-    CgSync* sync = nullptr;
+    mhd_host::SolveSync* sync = nullptr;
     double* partials = nullptr;
     double* dot_partial = nullptr;
     double* geta = nullptr;  // device accumulator of dL/deta
     double* host_small = nullptr;
     SweepGeom sg[2]{}, fg{};
     int st_blocks[2]{}, fn_blocks = 0;
-    int cg_strips_x = 0, cg_seg_h = 0, cg_nwarps = 0, cg_grid = 0;
+    mhd_host::SolveGeom geom;  // implicit solve
     int ew_blocks = 0, dot_blocks = 0;
     bool have_forward = false;
 };
@@ -137,7 +137,6 @@ mhd_status upload_coeffs(mhd_adjoint* a) {
 
 // (I - alpha L) x = rhs_scale * Jz(bxf, byf) with the step's alpha.
 mhd_status solve(mhd_adjoint* a, const double* bxf, const double* byf, double rhs_scale, double* x) {
-    MHD_TRY(cudaMemsetAsync(a->sync, 0, sizeof(CgSync), a->stream));
     CgSweepArgs g{};
     g.D = a->dom;
     g.D.eta = rhs_scale;
@@ -150,28 +149,14 @@ mhd_status solve(mhd_adjoint* a, const double* bxf, const double* byf, double rh
     g.p[0] = a->s.p[0];
     g.p[1] = a->s.p[1];
     g.partials = a->partials;
-    g.sync = a->sync;
     g.st = a->status;
     g.prods_out = nullptr;
     g.solve_index = 0;
-    g.strips_x = a->cg_strips_x;
-    g.seg_h = a->cg_seg_h;
-    g.nwarps = a->cg_nwarps;
     g.max_iters = a->prm.cg_max_iters > 0 ? a->prm.cg_max_iters : 2LL * (long long)a->n;
     g.tol = a->prm.cg_tol > 0 ? a->prm.cg_tol : 2.220446049250313e-16;
     g.timeout_s = a->prm.cg_timeout_s;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(a->cg_grid);
-    cfg.blockDim = dim3(CGS_NT);
-    cfg.dynamicSmemBytes = kCgRingBytes;
-    cfg.stream = a->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MHD_TRY(cudaLaunchKernelEx(&cfg, k_cg_sweep, g));
-    return MHD_OK;
+    return mhd_host::launch_solve(g, a->geom, mhd_host::solve_t((a->dt * a->eta) * a->g, a->prm.dx, a->prm.dy), a->sync,
+                                  a->stream);
 }
 
 // One forward step from U into slot sl (U^{n+1} = (sl.A[0..3], sl.Bn)) with the corner fields of
@@ -189,7 +174,6 @@ mhd_status forward_step(mhd_adjoint* a, const double* const U[6], const Slot& sl
         D, a->coeffs, cplanes6(sl.T), x1, planes6(sl.T), planes6(sl.A), a->sg[1]);
     MHD_TRY(cudaGetLastError());
     if (do_solve && (s = solve(a, sl.A[4], sl.A[5], a->eta, x2)) != MHD_OK) return s;
-    MHD_TRY(cudaMemsetAsync(&a->status->smax_bits, 0, sizeof(unsigned long long), a->stream));
     k_finalize_sweep<<<a->fn_blocks, 32 * FS_WARPS, 0, a->stream>>>(
         D, a->coeffs, planes6(sl.A), x2, sl.Bn[0], sl.Bn[1], a->status, a->fg);
     MHD_TRY(cudaGetLastError());
@@ -331,7 +315,10 @@ mhd_status read_status(mhd_adjoint* a) {
     DeviceStatus st;
     MHD_TRY(cudaMemcpy(&st, a->status, sizeof(st), cudaMemcpyDeviceToHost));
     if (st.flags) MHD_TRY(cudaMemset(&a->status->flags, 0, sizeof(unsigned int)));
-    if (st.flags & kStatusTimeout) return MHD_ERR_TIMEOUT;
+    if (st.flags & kStatusTimeout) {
+        MHD_TRY(cudaMemset(a->sync, 0, sizeof(*a->sync)));
+        return MHD_ERR_TIMEOUT;
+    }
     if (st.flags & kStatusNonFinite) return MHD_ERR_NONFINITE;
     if (st.flags & kStatusCgNotConverged) return MHD_ERR_CG_NOT_CONVERGED;
     return MHD_OK;
@@ -428,23 +415,8 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
         g.nwarps = g.strips_x * g.segs_y;
         a->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;
     }
-    {
-        int occ = 0;
-        if (cudaFuncSetAttribute(k_cg_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kCgRingBytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_sweep, CGS_NT, kCgRingBytes) !=
-                cudaSuccess || occ < 1)
-            return fail(MHD_ERR_CUDA);
-        a->cg_strips_x = (p->nx + CG_W - 1) / CG_W;
-        const long long rows_total = (long long)a->cg_strips_x * p->ny;
-        const long long max_blocks =
-            std::max(1LL, (rows_total + (CGS_NT / 32) * 4 - 1) / ((CGS_NT / 32) * 4));
-        a->cg_grid = (int)std::max(1LL, std::min((long long)a->num_sms, max_blocks));
-        const long long warps = (long long)a->cg_grid * (CGS_NT / 32);
-        const int segs = (int)std::max(1LL, warps / a->cg_strips_x);
-        a->cg_seg_h = std::max(4, (p->ny + segs - 1) / segs);
-        a->cg_nwarps = a->cg_strips_x * ((p->ny + a->cg_seg_h - 1) / a->cg_seg_h);
-    }
+    if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
+    a->geom = mhd_host::solve_geometry(p->nx, p->ny, a->num_sms);
     a->ew_blocks = std::max(1, std::min((int)((a->n + 255) / 256), a->num_sms * 8));
     a->dot_blocks = std::max(1, std::min((int)((a->n + 255) / 256), a->num_sms * 2));
     // memory: checkpoints, slots, scratch
@@ -454,8 +426,8 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
     if (cudaMalloc(&a->pool, planes * a->n * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&a->coeffs, sizeof(StepCoeffs)) != cudaSuccess ||
         cudaMalloc(&a->status, sizeof(DeviceStatus)) != cudaSuccess ||
-        cudaMalloc(&a->sync, sizeof(CgSync)) != cudaSuccess ||
-        cudaMalloc(&a->partials, (size_t)2 * a->cg_grid * 4 * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&a->sync, sizeof(*a->sync)) != cudaSuccess ||
+        cudaMalloc(&a->partials, a->geom.partials() * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&a->dot_partial, (size_t)a->dot_blocks * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&a->geta, sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&a->host_small, 8 * sizeof(double)) != cudaSuccess) {
@@ -500,6 +472,7 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
     s.bc[0] = take();
     s.bc[1] = take();
     if (cudaMemsetAsync(a->pool, 0, planes * a->n * sizeof(double), a->stream) != cudaSuccess ||
+        cudaMemsetAsync(a->sync, 0, sizeof(*a->sync), a->stream) != cudaSuccess ||
         cudaMemsetAsync(a->status, 0, sizeof(DeviceStatus), a->stream) != cudaSuccess)
         return fail(MHD_ERR_CUDA);
     const mhd_status st = upload_coeffs(a);

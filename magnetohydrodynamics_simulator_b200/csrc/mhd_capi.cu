@@ -19,7 +19,7 @@
 #include <vector>
 
 #include "../../include/mhd_b200.h"
-#include "mhd_cg_sweep.cuh"
+#include "mhd_solve.h"
 #include "mhd_snapshot.h"
 #include "mhd_host_util.h"
 #include "mhd_kernels.cuh"
@@ -56,7 +56,7 @@ struct mhd_context {
     double* r[2]{};
     double* p[2]{};
     double* partials = nullptr;
-    CgSync* sync = nullptr;
+    mhd_host::SolveSync* sync = nullptr;
     DeviceStatus* status = nullptr;
     StepCoeffs* coeffs = nullptr;
     double* divb_partial = nullptr;
@@ -69,7 +69,7 @@ struct mhd_context {
     int st_blocks[2]{};
     SweepGeom fg{};          // finalize sweep geometry
     int fn_blocks = 0;
-    int cg_strips_x = 0, cg_seg_h = 0, cg_nwarps = 0, cg_grid = 0;
+    mhd_host::SolveGeom solve;  // implicit solve
     bool have_state = false;
     bool alpha_fixed = false;
     double alpha = 0.0;
@@ -105,9 +105,9 @@ mhd_status launch_coeffs(mhd_context* c, double dt, int alpha_mode, double t_end
     return MHD_OK;
 }
 
-mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int solve_index,
+// t: the solve's t where the host knows it, else negative (mhd_host::launch_solve).
+mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int solve_index, double t,
                      long long* prods_out) {
-    MHD_TRY(cudaMemsetAsync(c->sync, 0, sizeof(CgSync), c->stream));
     CgSweepArgs a{};
     a.D = c->dom;
     a.C = c->coeffs;
@@ -119,28 +119,21 @@ mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int s
     a.p[0] = c->p[0];
     a.p[1] = c->p[1];
     a.partials = c->partials;
-    a.sync = c->sync;
     a.st = c->status;
     a.prods_out = prods_out;
     a.solve_index = solve_index;
-    a.strips_x = c->cg_strips_x;
-    a.seg_h = c->cg_seg_h;
-    a.nwarps = c->cg_nwarps;
     a.max_iters = c->prm.cg_max_iters > 0 ? c->prm.cg_max_iters : 2LL * (long long)c->n;
     a.tol = c->prm.cg_tol > 0 ? c->prm.cg_tol : 2.220446049250313e-16;
     a.timeout_s = c->prm.cg_timeout_s;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(c->cg_grid);
-    cfg.blockDim = dim3(CGS_NT);
-    cfg.dynamicSmemBytes = kCgRingBytes;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MHD_TRY(cudaLaunchKernelEx(&cfg, k_cg_sweep, a));
-    return MHD_OK;
+    return mhd_host::launch_solve(a, c->solve, t, c->sync, c->stream);
+}
+
+// t of a step's solves for the given dt; negative for a CFL step, whose dt the device chooses. (A run's
+// t_end can only shorten dt.)
+double step_t(const mhd_context* c, double dt) {
+    if (c->alpha_fixed) return mhd_host::solve_t(c->alpha, c->prm.dx, c->prm.dy);
+    if (c->prm.eta == 0.0) return 0.0;
+    return dt > 0.0 ? mhd_host::solve_t(dt * c->prm.eta * c->g, c->prm.dx, c->prm.dy) : -1.0;
 }
 
 CPlanes cplanes(double* const* f) {
@@ -173,22 +166,22 @@ mhd_status mark(mhd_context* c) {
     } while (0)
 
 // The kernels of one step after the coefficients kernel.
-mhd_status enqueue_step_body(mhd_context* c, long long* prods_out) {
+mhd_status enqueue_step_body(mhd_context* c, double dt, long long* prods_out) {
+    const double t = step_t(c, dt);
     MHD_MARK(c);
     k_stage_sweep<1><<<c->st_blocks[0], 32 * SW_WARPS, sweep_smem_bytes(1), c->stream>>>(
         c->dom, c->coeffs, cplanes(c->S), nullptr, planes(c->T), planes(c->A), c->sg[0]);
     MHD_TRY(cudaGetLastError());
     MHD_MARK(c);
-    mhd_status s = launch_cg(c, c->T[4], c->T[5], 0, prods_out);
+    mhd_status s = launch_cg(c, c->T[4], c->T[5], 0, t, prods_out);
     if (s != MHD_OK) return s;
     MHD_MARK(c);
     k_stage_sweep<2><<<c->st_blocks[1], 32 * SW_WARPS, sweep_smem_bytes(2), c->stream>>>(
         c->dom, c->coeffs, cplanes(c->T), c->x, planes(c->T), planes(c->A), c->sg[1]);
     MHD_TRY(cudaGetLastError());
     MHD_MARK(c);
-    s = launch_cg(c, c->A[4], c->A[5], 1, prods_out);
+    s = launch_cg(c, c->A[4], c->A[5], 1, t, prods_out);
     if (s != MHD_OK) return s;
-    MHD_TRY(cudaMemsetAsync(&c->status->smax_bits, 0, sizeof(unsigned long long), c->stream));
     MHD_MARK(c);
     k_finalize_sweep<<<c->fn_blocks, 32 * FS_WARPS, 0, c->stream>>>(
         c->dom, c->coeffs, planes(c->A), c->x, c->S[4], c->S[5], c->status, c->fg);
@@ -396,27 +389,8 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
         g.nwarps = g.strips_x * g.segs_y;
         c->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;
     }
-    // Implicit solve: one wave of co-resident blocks; strips of 32 corner columns split into row
-    // segments over all of their warps.
-    {
-        int occ = 0;
-        if (cudaFuncSetAttribute(k_cg_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kCgRingBytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_sweep, CGS_NT, kCgRingBytes) !=
-                cudaSuccess ||
-            occ < 1)
-            return fail(MHD_ERR_CUDA);
-        const int per_sm = std::max(1, std::min(occ, env_int("MHD_B200_CG_BLOCKS_PER_SM", 1)));
-        c->cg_strips_x = (p->nx + CG_W - 1) / CG_W;
-        const long long rows_total = (long long)c->cg_strips_x * p->ny;
-        // no more blocks than there are rows of work for their warps
-        const long long max_blocks = std::max(1LL, (rows_total + (CGS_NT / 32) * 4 - 1) / ((CGS_NT / 32) * 4));
-        c->cg_grid = (int)std::max(1LL, std::min((long long)per_sm * c->num_sms, max_blocks));
-        const long long warps = (long long)c->cg_grid * (CGS_NT / 32);
-        const int segs = (int)std::max(1LL, warps / c->cg_strips_x);
-        c->cg_seg_h = std::max(4, (p->ny + segs - 1) / segs);
-        c->cg_nwarps = c->cg_strips_x * ((p->ny + c->cg_seg_h - 1) / c->cg_seg_h);
-    }
+    if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
+    c->solve = mhd_host::solve_geometry(p->nx, p->ny, c->num_sms);
     c->divb_blocks = std::max(1, std::min((int)((c->n + 255) / 256), c->num_sms * 4));
     // memory
     if (cudaMalloc(&c->pool, (size_t)kPlanes * c->n * sizeof(double)) != cudaSuccess) {
@@ -435,8 +409,8 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
     c->r[1] = q + 2 * c->n;
     c->p[0] = q + 3 * c->n;
     c->p[1] = q + 4 * c->n;
-    if (cudaMalloc(&c->partials, (size_t)2 * c->cg_grid * 4 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&c->sync, sizeof(CgSync)) != cudaSuccess ||
+    if (cudaMalloc(&c->partials, c->solve.partials() * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&c->sync, sizeof(*c->sync)) != cudaSuccess ||
         cudaMalloc(&c->status, sizeof(DeviceStatus)) != cudaSuccess ||
         cudaMalloc(&c->coeffs, sizeof(StepCoeffs)) != cudaSuccess ||
         cudaMalloc(&c->divb_partial, (size_t)2 * c->divb_blocks * sizeof(double)) != cudaSuccess ||
@@ -447,6 +421,7 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
     }
     if (cudaMemsetAsync(c->status, 0, sizeof(DeviceStatus), c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->coeffs, 0, sizeof(StepCoeffs), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->sync, 0, sizeof(*c->sync), c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->pool, 0, (size_t)kPlanes * c->n * sizeof(double), c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
         return fail(MHD_ERR_CUDA);
@@ -691,7 +666,7 @@ mhd_status mhd_step(mhd_context* c, double dt) {
     if (!std::isfinite(dt)) return MHD_ERR_INVALID_ARGUMENT;
     s = launch_coeffs(c, dt, c->alpha_fixed ? 0 : 1, 0.0, nullptr);
     if (s != MHD_OK) return s;
-    return enqueue_step_body(c, nullptr);
+    return enqueue_step_body(c, dt, nullptr);
 }
 
 mhd_status mhd_run(mhd_context* c, int nsteps, double dt_fixed, double t_end, double* dts_out,
@@ -726,7 +701,7 @@ mhd_status mhd_run(mhd_context* c, int nsteps, double dt_fixed, double t_end, do
     auto one_step = [&]() -> mhd_status {
         mhd_status r = launch_coeffs(c, dt_fixed, mode, t_end, c->run.dts);
         if (r != MHD_OK) return r;
-        return enqueue_step_body(c, c->run.prods);
+        return enqueue_step_body(c, dt_fixed, c->run.prods);
     };
     // Two consecutive steps form one CUDA graph (the state's hydro planes swap every step, so
     // a pair returns to the same buffer assignment); it is replayed nsteps/2 times.
@@ -790,7 +765,7 @@ mhd_status mhd_resistive_rate(mhd_context* c, int solve_implicitly, double alpha
     if (solve_implicitly) {
         k_set_alpha<<<1, 1, 0, c->stream>>>(c->coeffs, alpha);
         MHD_TRY(cudaGetLastError());
-        s = launch_cg(c, bxf, byf, 0, nullptr);
+        s = launch_cg(c, bxf, byf, 0, mhd_host::solve_t(alpha, c->prm.dx, c->prm.dy), nullptr);
         if (s != MHD_OK) return s;
         k_corner_rates<<<blocks, 256, 0, c->stream>>>(c->dom, c->x, nullptr, nullptr, bx_rate, by_rate);
     } else {
@@ -911,6 +886,7 @@ mhd_status mhd_synchronize(mhd_context* c) {
     memcpy(&st, c->host_pinned, sizeof(st));
     if (st.flags) {
         MHD_TRY(cudaMemsetAsync(&c->status->flags, 0, sizeof(unsigned int), c->stream));
+        if (st.flags & kStatusTimeout) MHD_TRY(cudaMemsetAsync(c->sync, 0, sizeof(*c->sync), c->stream));
         MHD_TRY(cudaStreamSynchronize(c->stream));
     }
     return status_from_flags(st.flags);
@@ -985,12 +961,12 @@ mhd_status mhd_cg_products_sum(mhd_context* c, long long out[2]) {
 namespace {
 
 constexpr size_t kNoAllocCells = MHD_NOALLOC_MAX_CELLS;
-constexpr int kNoAllocMaxBlocks = 1024;
+constexpr int kNoAllocMaxBlocks = 256;
 constexpr size_t kNoAllocVecDoubles = 5 * kNoAllocCells;             // x, r0, r1, p0, p1
-constexpr size_t kNoAllocPartialDoubles = 2 * 4 * (size_t)kNoAllocMaxBlocks;
-constexpr size_t kNoAllocControlDoubles = 64;                        // CgSync, DeviceStatus, StepCoeffs
+constexpr size_t kNoAllocPartialDoubles = (CM_NMU + 8) * (size_t)kNoAllocMaxBlocks;
+constexpr size_t kNoAllocControlDoubles = 64;                        // SolveSync, DeviceStatus, StepCoeffs
 constexpr size_t kNoAllocDoubles = kNoAllocVecDoubles + kNoAllocPartialDoubles + kNoAllocControlDoubles;
-static_assert(sizeof(CgSync) + sizeof(DeviceStatus) + sizeof(StepCoeffs) <= 8 * kNoAllocControlDoubles,
+static_assert(sizeof(mhd_host::SolveSync) + sizeof(DeviceStatus) + sizeof(StepCoeffs) <= 8 * kNoAllocControlDoubles,
               "control blocks exceed their reserved space");
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
@@ -1012,12 +988,10 @@ mhd_status noalloc_setup(int dev, NoAllocDevice** out) {
     if (!d.ready) {
         void* addr = nullptr;
         MHD_TRY(cudaGetSymbolAddress(&addr, g_noalloc_scratch));
-        MHD_TRY(cudaFuncSetAttribute(k_cg_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kCgRingBytes));
-        int occ = 0, sms = 0;
-        MHD_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_sweep, CGS_NT, kCgRingBytes));
+        int sms = 0;
         MHD_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        if (occ < 1) return MHD_ERR_CUDA;
+        const mhd_status s = mhd_host::solve_setup();
+        if (s != MHD_OK) return s;
         d.scratch = static_cast<double*>(addr);
         // one block per SM, as a context launches the solver
         d.grid = std::max(1, std::min(sms, kNoAllocMaxBlocks));
@@ -1065,27 +1039,19 @@ extern "C" mhd_status mhd_resistive_rate_noalloc(const mhd_params* p, int solve_
     double* p1 = base + 4 * kNoAllocCells;
     double* partials = base + kNoAllocVecDoubles;
     unsigned char* ctrl = reinterpret_cast<unsigned char*>(partials + kNoAllocPartialDoubles);
-    CgSync* sync = reinterpret_cast<CgSync*>(ctrl);
-    DeviceStatus* st = reinterpret_cast<DeviceStatus*>(ctrl + 64);
-    StepCoeffs* coeffs = reinterpret_cast<StepCoeffs*>(ctrl + 64 + 128);
-    static_assert(sizeof(CgSync) <= 64 && sizeof(DeviceStatus) <= 128 &&
-                      64 + 128 + sizeof(StepCoeffs) <= 8 * kNoAllocControlDoubles,
+    mhd_host::SolveSync* sync = reinterpret_cast<mhd_host::SolveSync*>(ctrl);
+    DeviceStatus* st = reinterpret_cast<DeviceStatus*>(ctrl + 128);
+    StepCoeffs* coeffs = reinterpret_cast<StepCoeffs*>(ctrl + 128 + 128);
+    static_assert(sizeof(mhd_host::SolveSync) <= 128 && sizeof(DeviceStatus) <= 128 &&
+                      128 + 128 + sizeof(StepCoeffs) <= 8 * kNoAllocControlDoubles,
                   "control block layout");
     // what must start at zero: the barrier counter, the status and the coefficient block (the
     // array keeps the previous call's contents)
     MHD_TRY(cudaMemsetAsync(ctrl, 0, 8 * kNoAllocControlDoubles, stream));
     k_set_alpha<<<1, 1, 0, stream>>>(coeffs, alpha);
     MHD_TRY(cudaGetLastError());
-    // solver geometry exactly as a context's (mhd_create): strips of CG_W columns, no more blocks
-    // than rows of work for their warps, so both entry points reduce in the same order
-    const int strips_x = (p->nx + CG_W - 1) / CG_W;
-    const long long rows_total = (long long)strips_x * p->ny;
-    const long long max_blocks =
-        std::max(1LL, (rows_total + (CGS_NT / 32) * 4 - 1) / ((CGS_NT / 32) * 4));
-    const int grid = (int)std::max(1LL, std::min((long long)nd->grid, max_blocks));
-    const long long warps = (long long)grid * (CGS_NT / 32);
-    const int segs = (int)std::max(1LL, warps / strips_x);
-    const int seg_h = std::max(4, (p->ny + segs - 1) / segs);
+    // solver geometry exactly as a context's (mhd_create), so both entry points reduce in the same order
+    const mhd_host::SolveGeom geom = mhd_host::solve_geometry(p->nx, p->ny, nd->grid);
     CgSweepArgs a{};
     a.D = D;
     a.C = coeffs;
@@ -1097,27 +1063,14 @@ extern "C" mhd_status mhd_resistive_rate_noalloc(const mhd_params* p, int solve_
     a.p[0] = p0;
     a.p[1] = p1;
     a.partials = partials;
-    a.sync = sync;
     a.st = st;
     a.prods_out = nullptr;
     a.solve_index = 0;
-    a.strips_x = strips_x;
-    a.seg_h = seg_h;
-    a.nwarps = strips_x * ((p->ny + seg_h - 1) / seg_h);
     a.max_iters = p->cg_max_iters > 0 ? p->cg_max_iters : 2LL * (long long)n;
     a.tol = p->cg_tol > 0 ? p->cg_tol : 2.220446049250313e-16;
     a.timeout_s = p->cg_timeout_s > 0 ? p->cg_timeout_s : 30.0;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(CGS_NT);
-    cfg.dynamicSmemBytes = kCgRingBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MHD_TRY(cudaLaunchKernelEx(&cfg, k_cg_sweep, a));
+    s = mhd_host::launch_solve(a, geom, mhd_host::solve_t(alpha, p->dx, p->dy), sync, stream);
+    if (s != MHD_OK) return s;
     k_corner_rates<<<blocks, 256, 0, stream>>>(D, x, nullptr, nullptr, bx_rate, by_rate);
     MHD_TRY(cudaGetLastError());
     // The solve's status lives only in the shared array, where the next call clears it, so it is

@@ -47,6 +47,7 @@ struct CgSweepArgs {
     double* p[2];
     double* partials;  // [2][gridDim.x][4]
     CgSync* sync;
+    struct CgStart* start;  // where k_cg_sweep, launched behind k_solve, enters (null: it is not)
     DeviceStatus* st;
     long long* prods_out;
     int solve_index;
@@ -64,6 +65,17 @@ struct CgScal {
     double cx, cy, diag;
     double alpha_prev;  // alpha_{k-1} (odd iterations fold its update of x into theirs)
 };
+
+__device__ __forceinline__ CgScal cg_scalars(const CgSweepArgs& a) {
+    CgScal s;
+    const double alpha_m = a.C->alpha;
+    s.cx = alpha_m / (a.D.dx * a.D.dx);
+    s.cy = alpha_m / (a.D.dy * a.D.dy);
+    s.diag = 1 + 2 * (s.cx + s.cy);
+    s.invdiag = (s.diag == 0.0) ? 1.0 : 1.0 / s.diag;
+    s.beta = s.alpha = s.alpha_prev = 0.0;
+    return s;
+}
 
 // How an iteration's sweep treats the solution x (see the header comment).
 enum CgXMode : int {
@@ -311,7 +323,7 @@ __device__ __forceinline__ void cg_iter_segment(const CgSweepArgs& a, const CgSc
 }
 
 // Block-reduce NV partial sums (fixed order) and publish them in this block's slot.
-template <int NV>
+template <int NV, int NT = CGS_NT>
 __device__ __forceinline__ void publish(double (&acc)[4], double* slot, double* red) {
 #pragma unroll
     for (int k = 0; k < NV; ++k)
@@ -325,83 +337,104 @@ __device__ __forceinline__ void publish(double (&acc)[4], double* slot, double* 
     __syncthreads();
     if (threadIdx.x < NV) {
         double sum = 0.0;
-        for (int q = 0; q < CGS_NT / 32; ++q) sum += red[q * 4 + threadIdx.x];
+        for (int q = 0; q < NT / 32; ++q) sum += red[q * 4 + threadIdx.x];
         slot[threadIdx.x] = sum;
     }
 }
 
-static __global__ void __launch_bounds__(CGS_NT, MHD_CG_MIN_BLOCKS)
-k_cg_sweep(CgSweepArgs a) {
-    __shared__ double red[CGS_NT / 32 * 4];
-    __shared__ double scal[8];
-    __shared__ int sflag;
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double cg_ring_mem[];
-#else
-    // host compilation of the kernel sources (single-block logic tests): one shared copy
-    static double cg_ring_mem[(CGS_NT / 32) * CG_RING * CG_SLOT];
-#endif
-    double* const ring = cg_ring_mem + (size_t)(threadIdx.x >> 5) * CG_RING * CG_SLOT;
+// One sweep of the whole grid on NT threads a block, as a function of its own for a kernel in which other
+// values would live across the inlined one: this warp's segments, then the block's sums.
+template <int NT, bool FIRST, int XM, bool RHS = false>
+static __device__ __noinline__ void cg_phase_call(const CgSweepArgs& a, int strips_x, int seg_h, int nwarps, CgScal s,
+                                                  int dir, const double* rk, const double* pkm1, double* rk1, double* pk,
+                                                  double* ring, double* partials, double* red) {
+    constexpr int NW = NT / 32;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int w = blockIdx.x * NW + (threadIdx.x >> 5); w < nwarps; w += gridDim.x * NW) {
+        const int sx = w % strips_x, r0w = (w / strips_x) * seg_h;
+        const int r1w = min(r0w + seg_h, a.D.ny);
+        if constexpr (RHS) cg_rhs_segment(a, s, sx, r0w, r1w, dir, rk1, ring, acc);
+        else cg_iter_segment<FIRST, XM>(a, s, sx, r0w, r1w, dir, rk, pkm1, rk1, pk, ring, acc);
+    }
+    publish<RHS ? 3 : 4, NT>(acc, partials + (size_t)blockIdx.x * 4, red);
+}
+
+// Where a solve enters its iterations: k = 0 is the right-hand side; k > 0 (odd) goes on from
+// r_k, p_{k-1} and x_{k-1} that the caller left in the buffers iteration k reads, with its scalars;
+// k < 0: nothing is left to do.
+struct CgStart {
+    long long k;
+    double alpha, alpha_prev, beta, absNew, pAp, bb, threshold;
+};
+struct CgResult {
+    long long products;
+    double bb, rr;
+    bool breakdown, converged;
+};
+
+// The iterations of the header comment on all warps of the grid, NT threads a block. barrier() is the
+// grid-wide barrier; false as soon as it gives up.
+// START: `start` may ask for a later iteration than the right-hand side. INLINE: the sweeps are inlined.
+template <int NT, bool INLINE, bool START, class Barrier>
+__device__ __forceinline__ bool cg_iterate(const CgSweepArgs& a, int strips_x, int seg_h, int nwarps, CgScal& s,
+                                           double* ring, double* partials, double* red, double* scal,
+                                           Barrier&& barrier, const CgStart& start, CgResult& res) {
     const int tid = threadIdx.x;
     const int G = gridDim.x;
-    const int warps_per_block = CGS_NT / 32;
-    const int wfirst = blockIdx.x * warps_per_block + (tid >> 5);
-    const int wstride = G * warps_per_block;
-    CgScal s;
-    const double alpha_m = a.C->alpha;
-    s.cx = alpha_m / (a.D.dx * a.D.dx);
-    s.cy = alpha_m / (a.D.dy * a.D.dy);
-    s.diag = 1 + 2 * (s.cx + s.cy);
-    s.invdiag = (s.diag == 0.0) ? 1.0 : 1.0 / s.diag;
-    s.beta = 0.0;
-    s.alpha = 0.0;
-    s.alpha_prev = 0.0;
-    unsigned long long target = 0;
-    const unsigned long long deadline =
-        global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
-    double* const part0 = a.partials;
-    double* const part1 = a.partials + (size_t)G * 4;
+    const int wfirst = blockIdx.x * (NT / 32) + (tid >> 5);
+    const int wstride = G * (NT / 32);
+    double* const part0 = partials;
+    double* const part1 = partials + (size_t)G * 4;
     // (conditional selects instead of indexing small arrays by a runtime value, which would put
     // them in local memory)
     auto part = [&](int ph) { return (ph & 1) ? part1 : part0; };
     int phase = 0;
     int dir = 1;
-
-    auto barrier_or_quit = [&]() -> bool {
-        if (grid_barrier(a.sync, target, deadline, &sflag)) return true;
-        if (tid == 0 && blockIdx.x == 0) atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
-        return false;
-    };
-
-    // ---- right-hand side: r0 = b, p0 = z0 = b/d; |b|^2, b.z0, p0.A p0
-    {
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int w = wfirst; w < a.nwarps; w += wstride) {
-            const int sx = w % a.strips_x, r0w = (w / a.strips_x) * a.seg_h;
-            cg_rhs_segment(a, s, sx, r0w, min(r0w + a.seg_h, a.D.ny), dir, a.r[0], ring, acc);
+    double bb, absNew, pAp, threshold;
+    bool zero_solution = false, breakdown = false, converged = false;
+    const long long k0 = START ? start.k : 0;
+    if (k0 == 0) {
+        // ---- right-hand side: r0 = b, p0 = z0 = b/d; |b|^2, b.z0, p0.A p0
+        if constexpr (INLINE) {
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int w = wfirst; w < nwarps; w += wstride) {
+                const int sx = w % strips_x, r0w = (w / strips_x) * seg_h;
+                cg_rhs_segment(a, s, sx, r0w, min(r0w + seg_h, a.D.ny), dir, a.r[0], ring, acc);
+            }
+            publish<3, NT>(acc, part(phase) + (size_t)blockIdx.x * 4, red);
+        } else {
+            cg_phase_call<NT, false, kXSkip, true>(a, strips_x, seg_h, nwarps, s, dir, nullptr, nullptr, a.r[0], nullptr,
+                                                   ring, part(phase), red);
         }
-        publish<3>(acc, part(phase) + (size_t)blockIdx.x * 4, red);
+        if (!barrier()) return false;
+        double sums[4];
+        reduce_partials<3>(part(phase), G, sums, scal);
+        ++phase;
+        dir = -dir;
+        bb = sums[0];
+        absNew = sums[1];
+        pAp = sums[2];
+        threshold = smax(a.tol * a.tol * bb, 2.2250738585072014e-308);
+        zero_solution = (bb == 0.0) || (bb < threshold);
+        breakdown = !isfinite(bb);
+        converged = zero_solution;
+        s.alpha = absNew / pAp;
+    } else {
+        bb = start.bb;
+        absNew = start.absNew;
+        pAp = start.pAp;
+        threshold = start.threshold;
+        s.alpha = start.alpha;
+        s.alpha_prev = start.alpha_prev;
+        s.beta = start.beta;
     }
-    if (!barrier_or_quit()) return;
-    double sums[4];
-    reduce_partials<3>(part(phase), G, sums, scal);
-    ++phase;
-    dir = -dir;
-    const double bb = sums[0];
-    double absNew = sums[1];
-    double pAp = sums[2];
-    const double threshold = smax(a.tol * a.tol * bb, 2.2250738585072014e-308);
-    long long products = 0;
-    const bool zero_solution = (bb == 0.0) || (bb < threshold);
-    bool breakdown = !isfinite(bb);
-    bool converged = zero_solution;
+    long long products = k0;
     double rr_final = 0.0;
     long long k_last = -1;     // the last iteration swept
     double alpha_last = 0.0;   // its step length
 
     if (!zero_solution && !breakdown) {
-        s.alpha = absNew / pAp;
-        for (long long k = 0; k < a.max_iters; ++k) {
+        for (long long k = k0; k < a.max_iters; ++k) {
             k_last = k;
             alpha_last = s.alpha;
             const bool odd = (k & 1) != 0;
@@ -409,11 +442,11 @@ k_cg_sweep(CgSweepArgs a) {
             double* rk1 = odd ? a.r[0] : a.r[1];
             const double* pkm1 = odd ? a.p[0] : a.p[1];
             double* pk = odd ? a.p[1] : a.p[0];
-            {
+            if constexpr (INLINE) {
                 double acc[4] = {0.0, 0.0, 0.0, 0.0};
-                for (int w = wfirst; w < a.nwarps; w += wstride) {
-                    const int sx = w % a.strips_x, r0w = (w / a.strips_x) * a.seg_h;
-                    const int r1w = min(r0w + a.seg_h, a.D.ny);
+                for (int w = wfirst; w < nwarps; w += wstride) {
+                    const int sx = w % strips_x, r0w = (w / strips_x) * seg_h;
+                    const int r1w = min(r0w + seg_h, a.D.ny);
                     switch (cg_xmode(k)) {
                         case kXSkip:
                             if (k == 0)
@@ -428,9 +461,27 @@ k_cg_sweep(CgSweepArgs a) {
                             cg_iter_segment<false, kXPair>(a, s, sx, r0w, r1w, dir, rk, pkm1, rk1, pk, ring, acc);
                     }
                 }
-                publish<4>(acc, part(phase) + (size_t)blockIdx.x * 4, red);
+                publish<4, NT>(acc, part(phase) + (size_t)blockIdx.x * 4, red);
+            } else {
+                switch (cg_xmode(k)) {
+                    case kXSkip:
+                        if (k == 0)
+                            cg_phase_call<NT, true, kXSkip>(a, strips_x, seg_h, nwarps, s, dir, rk, pkm1, rk1, pk, ring,
+                                                            part(phase), red);
+                        else
+                            cg_phase_call<NT, false, kXSkip>(a, strips_x, seg_h, nwarps, s, dir, rk, pkm1, rk1, pk, ring,
+                                                             part(phase), red);
+                        break;
+                    case kXPairFirst:
+                        cg_phase_call<NT, false, kXPairFirst>(a, strips_x, seg_h, nwarps, s, dir, rk, pkm1, rk1, pk, ring,
+                                                              part(phase), red);
+                        break;
+                    default:
+                        cg_phase_call<NT, false, kXPair>(a, strips_x, seg_h, nwarps, s, dir, rk, pkm1, rk1, pk, ring,
+                                                         part(phase), red);
+                }
             }
-            if (!barrier_or_quit()) return;
+            if (!barrier()) return false;
             double v[4];
             reduce_partials<4>(part(phase), G, v, scal);
             ++phase;
@@ -454,24 +505,66 @@ k_cg_sweep(CgSweepArgs a) {
         // the last iteration was even: add its alpha_k p_k (x_0 = 0 when it was the first)
         const double* pl = (k_last & 1) ? a.p[1] : a.p[0];
         const size_t n = (size_t)a.D.nx * a.D.ny;
-        for (size_t g = (size_t)blockIdx.x * CGS_NT + tid; g < n; g += (size_t)G * CGS_NT)
+        for (size_t g = (size_t)blockIdx.x * NT + tid; g < n; g += (size_t)G * NT)
             a.x[g] = (k_last == 0) ? alpha_last * pl[g] : fma(alpha_last, pl[g], a.x[g]);
     }
     if (zero_solution || breakdown || k_last < 0) {
         // x = 0 (Eigen returns the zero vector when b == 0, and x0 = 0 when no iteration may run);
         // on breakdown the status says so
-        const int nx = a.D.nx, ny = a.D.ny;
-        const size_t n = (size_t)nx * ny;
-        for (size_t g = (size_t)blockIdx.x * CGS_NT + tid; g < n; g += (size_t)G * CGS_NT) a.x[g] = 0.0;
+        const size_t n = (size_t)a.D.nx * a.D.ny;
+        for (size_t g = (size_t)blockIdx.x * NT + tid; g < n; g += (size_t)G * NT) a.x[g] = 0.0;
     }
-    if (blockIdx.x == 0 && tid == 0) {
-        a.st->cg_products[a.solve_index] = products;
-        a.st->cg_products_sum[a.solve_index] += products;
-        a.st->cg_last_rr[a.solve_index] = (bb > 0.0) ? rr_final / bb : 0.0;
-        if (a.prods_out) a.prods_out[2 * a.C->cur + a.solve_index] = products;
-        if (breakdown) atomicOr(&a.st->flags, (unsigned)(kStatusCgBreakdown | kStatusNonFinite));
-        else if (!converged) atomicOr(&a.st->flags, (unsigned)kStatusCgNotConverged);
+    res.products = products;
+    res.bb = bb;
+    res.rr = rr_final;
+    res.breakdown = breakdown;
+    res.converged = converged;
+    return true;
+}
+
+// A solve's outcome in the device status (one thread).
+__device__ __forceinline__ void cg_report(const CgSweepArgs& a, const CgResult& r) {
+    a.st->cg_products[a.solve_index] = r.products;
+    a.st->cg_products_sum[a.solve_index] += r.products;
+    a.st->cg_last_rr[a.solve_index] = (r.bb > 0.0) ? r.rr / r.bb : 0.0;
+    if (a.prods_out) a.prods_out[2 * a.C->cur + a.solve_index] = r.products;
+    if (r.breakdown) atomicOr(&a.st->flags, (unsigned)(kStatusCgBreakdown | kStatusNonFinite));
+    else if (!r.converged) atomicOr(&a.st->flags, (unsigned)kStatusCgNotConverged);
+}
+
+// START: behind k_solve, which says in a.start what is left to do.
+template <bool START>
+__global__ void __launch_bounds__(CGS_NT, MHD_CG_MIN_BLOCKS)
+k_cg_sweep(const __grid_constant__ CgSweepArgs a) {
+    __shared__ double red[CGS_NT / 32 * 4];
+    __shared__ double scal[8];
+    __shared__ int sflag;
+#if defined(__CUDA_ARCH__)
+    extern __shared__ __align__(16) double cg_ring_mem[];
+#else
+    // host compilation of the kernel sources (single-block logic tests): one shared copy
+    static double cg_ring_mem[(CGS_NT / 32) * CG_RING * CG_SLOT];
+#endif
+    CgStart start{};
+    if constexpr (START) {
+        start = *a.start;
+        if (start.k < 0) return;
     }
+    double* const ring = cg_ring_mem + (size_t)(threadIdx.x >> 5) * CG_RING * CG_SLOT;
+    const int tid = threadIdx.x;
+    CgScal s = cg_scalars(a);
+    unsigned long long target = barrier_base(a.sync);
+    const unsigned long long deadline =
+        global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
+    auto barrier = [&]() -> bool {
+        if (grid_barrier(a.sync, target, deadline, &sflag)) return true;
+        // (any block: one that gives up leaves its part undone)
+        if (tid == 0) atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
+        return false;
+    };
+    CgResult res{};
+    if (cg_iterate<CGS_NT, true, START>(a, a.strips_x, a.seg_h, a.nwarps, s, ring, a.partials, red, scal, barrier, start, res) && blockIdx.x == 0 && tid == 0)
+        cg_report(a, res);
 }
 
 }  // namespace mhd

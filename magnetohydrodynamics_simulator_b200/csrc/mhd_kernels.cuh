@@ -78,8 +78,8 @@ struct DeviceStatus {
 };
 
 struct CgSync {
-    unsigned long long count;  // zeroed before each launch of the solver
-    unsigned int error;
+    unsigned long long count;  // arrivals: zero at a launch, or a multiple of the grid (see barrier_base)
+    unsigned int error;        // a wait ran out of time
     unsigned int pad;
 };
 
@@ -205,6 +205,15 @@ __device__ __forceinline__ bool grid_barrier(CgSync* sync, unsigned long long& t
     return *sflag != 0;
 }
 
+// The barrier target to start from where the counter is not zeroed between launches (thread 0's value
+// counts): launches that completed their barriers left a multiple of the grid, and no block passes the
+// first barrier of this launch before this one has arrived there.
+__device__ __forceinline__ unsigned long long barrier_base(const CgSync* sync) {
+    if (threadIdx.x != 0) return 0;
+    const unsigned long long c = *(const volatile unsigned long long*)&sync->count;
+    return c - c % gridDim.x;
+}
+
 // This lane's sum of K consecutive doubles of the 4-double partials of blocks lane, lane + 32, ...
 // (< nblocks), in that order. The loads of four blocks are issued before they are added, so a lane
 // waits for one round trip per four blocks instead of one per block; the sum is the same.
@@ -305,11 +314,13 @@ __device__ __forceinline__ void step_coeffs_one(StepCoeffs* C, const DeviceStatu
     C->t += dt;
 }
 
-static __global__ void k_step_coeffs(StepCoeffs* C, const DeviceStatus* st, double dt, double alpha,
+// (Also zeroes the max signal speed, which this step's finalize forms anew.)
+static __global__ void k_step_coeffs(StepCoeffs* C, DeviceStatus* st, double dt, double alpha,
                               int alpha_mode, double eta, double hmin, double courant,
                               double safety, double g, double d, double t_end, double* dts_out) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     step_coeffs_one(C, st, dt, alpha, alpha_mode, eta, hmin, courant, safety, g, d, t_end, dts_out);
+    st->smax_bits = 0ULL;
 }
 
 // ------------------------------------------------------------------------------------------
