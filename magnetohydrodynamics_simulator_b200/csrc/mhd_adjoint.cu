@@ -174,7 +174,7 @@ mhd_status forward_step(mhd_adjoint* a, const double* const U[6], const Slot& sl
         D, a->coeffs, cplanes6(sl.T), x1, planes6(sl.T), planes6(sl.A), a->sg[1]);
     MHD_TRY(cudaGetLastError());
     if (do_solve && (s = solve(a, sl.A[4], sl.A[5], a->eta, x2)) != MHD_OK) return s;
-    k_finalize_sweep<<<a->fn_blocks, 32 * FS_WARPS, 0, a->stream>>>(
+    k_finalize_sweep<<<a->fn_blocks, 32 * FS_WARPS, kFinSmemBytes, a->stream>>>(
         D, a->coeffs, planes6(sl.A), x2, sl.Bn[0], sl.Bn[1], a->status, a->fg);
     MHD_TRY(cudaGetLastError());
     return MHD_OK;
@@ -396,21 +396,21 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
         SweepGeom& g = a->sg[mode];
         g.strips_x = (p->nx + SW_OUT - 1) / SW_OUT;
         const int segs = (int)std::max(1LL, resident / g.strips_x);
-        g.seg_h = std::max(16, (p->ny + segs - 1) / segs);
+        g.seg_h = std::max(3, (p->ny + segs - 1) / segs);
         g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
         g.nwarps = g.strips_x * g.segs_y;
         a->st_blocks[mode] = (g.nwarps + SW_WARPS - 1) / SW_WARPS;
     }
     {
         int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, kFinSmemBytes) !=
                 cudaSuccess || occ < 1)
             return fail(MHD_ERR_CUDA);
         const long long resident = (long long)occ * a->num_sms * FS_WARPS;
         SweepGeom& g = a->fg;
         g.strips_x = (p->nx + FS_OUT - 1) / FS_OUT;
         const int segs = (int)std::max(1LL, resident / g.strips_x);
-        g.seg_h = std::max(16, (p->ny + segs - 1) / segs);
+        g.seg_h = std::max(3, (p->ny + segs - 1) / segs);
         g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
         g.nwarps = g.strips_x * g.segs_y;
         a->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;

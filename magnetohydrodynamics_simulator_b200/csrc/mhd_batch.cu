@@ -167,7 +167,7 @@ mhd_status apply_tuning(mhd_batch* b, const mhd_batch_tuning& t) {
     MHD_TRY(cudaStreamSynchronize(b->stream));  // in-flight steps still read the old lists
     std::vector<SweepItem> st_items, fin_items;
     strip_items(b, t.stage_rows, t.stage_tail_rows, st_items);
-    strip_items(b, std::max(16, balanced_rows(b, (long long)b->fin_occ * b->num_sms * FS_WARPS, 1)), 0,
+    strip_items(b, std::max(3, balanced_rows(b, (long long)b->fin_occ * b->num_sms * FS_WARPS, 1)), 0,
                 fin_items);
     // solver: its grid covers the largest chunk at 8 or more rows per warp
     for (int p = 0; p < 2; ++p)
@@ -266,7 +266,7 @@ mhd_status enqueue_step(mhd_batch* b, const double* dt_in, double dt_fixed, int 
     s = launch_cg_chunks(b, I, 1, record);
     if (s != MHD_OK) return s;
     if (ev) MHD_TRY(cudaEventRecord(ev[4], b->stream));
-    k_finalize_batch<<<b->fin_grid, 32 * FS_WARPS, 0, b->stream>>>(I, b->d_fin_items, b->n_fin_items,
+    k_finalize_batch<<<b->fin_grid, 32 * FS_WARPS, kFinSmemBytes, b->stream>>>(I, b->d_fin_items, b->n_fin_items,
                                                                    b->queues + 2, b->fin_base[b->parity]);
     MHD_TRY(cudaGetLastError());
     if (ev) MHD_TRY(cudaEventRecord(ev[5], b->stream));
@@ -361,7 +361,7 @@ mhd_status mhd_batch_create(const mhd_params* params, int count, void* stream, m
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->stage_occ[1], k_stage_batch<2>,
                                                       32 * SW_WARPS, sweep_smem_bytes(2)) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->fin_occ, k_finalize_batch, 32 * FS_WARPS,
-                                                      0) != cudaSuccess ||
+                                                      kFinSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(k_cg_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kCgbSmemBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->cg_occ, k_cg_batch, CGB_NT, kCgbSmemBytes) !=

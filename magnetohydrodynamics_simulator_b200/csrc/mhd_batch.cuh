@@ -110,7 +110,7 @@ k_stage_batch(const BatchInst* __restrict__ insts, const SweepItem* __restrict__
 #if defined(__CUDA_ARCH__)
     extern __shared__ __align__(16) double sw_ring_mem[];
 #else
-    static double sw_ring_mem[SW_WARPS * (SW_RING * SW_SLOT + SW_CARRY)];
+    static double sw_ring_mem[SW_WARPS * (sweep_warp_doubles(1) + sweep_warp_doubles(2))];
 #endif
     __shared__ SweepInstRec rec[SW_WARPS];
     const int wl = threadIdx.x >> 5;
@@ -128,7 +128,7 @@ k_stage_batch(const BatchInst* __restrict__ insts, const SweepItem* __restrict__
         }
         __syncwarp();
         stage_sweep_warp<MODE, RecPlanes, MODE == 1 ? MHD_SWEEP_YREUSE_1 : MHD_BATCH_YREUSE_2,
-                         MODE == 1 ? MHD_SWEEP_XREUSE_1 : MHD_BATCH_XREUSE_2, MODE == 1>(
+                         MODE == 1 ? MHD_SWEEP_XREUSE_1 : MHD_BATCH_XREUSE_2>(
             I.C, pl, e.sx, e.r0, e.r1, ring);
     }
 }
@@ -152,9 +152,14 @@ struct RecFin {
 
 // Finalize of the batch. base: the arenas of this step's parity (acc = accumulator, x = E2,
 // bx / by = the state's face planes).
-static __global__ void __launch_bounds__(32 * FS_WARPS)
+static __global__ void __launch_bounds__(32 * FS_WARPS, kFinMinBlocks)
 k_finalize_batch(const BatchInst* __restrict__ insts, const SweepItem* __restrict__ items, int nitems,
                  int* queue, FinParams base) {
+#if defined(__CUDA_ARCH__)
+    extern __shared__ __align__(16) double fs_ring_mem[];
+#else
+    static double fs_ring_mem[FS_WARPS * FS_RING * FS_SLOT];
+#endif
     __shared__ SweepInstRec rec[FS_WARPS];
     const int wl = threadIdx.x >> 5;
     const RecFin f{base, &rec[wl]};
@@ -169,7 +174,7 @@ k_finalize_batch(const BatchInst* __restrict__ insts, const SweepItem* __restric
             rec[wl].off = I.off;
         }
         __syncwarp();
-        finalize_sweep_warp(f, I.C, I.st, e.sx, e.r0, e.r1);
+        finalize_sweep_warp(f, I.C, I.st, e.sx, e.r0, e.r1, fs_ring_mem + (size_t)wl * FS_RING * FS_SLOT);
     }
 }
 

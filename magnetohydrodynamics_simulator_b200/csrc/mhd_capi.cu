@@ -183,7 +183,7 @@ mhd_status enqueue_step_body(mhd_context* c, double dt, long long* prods_out) {
     s = launch_cg(c, c->A[4], c->A[5], 1, t, prods_out);
     if (s != MHD_OK) return s;
     MHD_MARK(c);
-    k_finalize_sweep<<<c->fn_blocks, 32 * FS_WARPS, 0, c->stream>>>(
+    k_finalize_sweep<<<c->fn_blocks, 32 * FS_WARPS, kFinSmemBytes, c->stream>>>(
         c->dom, c->coeffs, planes(c->A), c->x, c->S[4], c->S[5], c->status, c->fg);
     MHD_TRY(cudaGetLastError());
     MHD_MARK(c);
@@ -366,7 +366,7 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
         SweepGeom& g = c->sg[mode];
         g.strips_x = (p->nx + SW_OUT - 1) / SW_OUT;
         const int segs = (int)std::max(1LL, resident / g.strips_x);
-        g.seg_h = std::max(env_int("MHD_B200_STAGE_MIN_ROWS", 16), (p->ny + segs - 1) / segs);
+        g.seg_h = std::max(env_int("MHD_B200_STAGE_MIN_ROWS", 3), (p->ny + segs - 1) / segs);
         g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
         g.nwarps = g.strips_x * g.segs_y;
         c->st_blocks[mode] = (g.nwarps + SW_WARPS - 1) / SW_WARPS;
@@ -376,7 +376,7 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
     }
     {
         int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, kFinSmemBytes) !=
                 cudaSuccess ||
             occ < 1)
             return fail(MHD_ERR_CUDA);
@@ -384,7 +384,7 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
         SweepGeom& g = c->fg;
         g.strips_x = (p->nx + FS_OUT - 1) / FS_OUT;
         const int segs = (int)std::max(1LL, resident / g.strips_x);
-        g.seg_h = std::max(16, (p->ny + segs - 1) / segs);
+        g.seg_h = std::max(3, (p->ny + segs - 1) / segs);
         g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
         g.nwarps = g.strips_x * g.segs_y;
         c->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;

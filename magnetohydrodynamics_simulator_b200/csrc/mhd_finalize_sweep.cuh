@@ -8,6 +8,10 @@
 // Lane l holds column c0 - 1 + l; outputs are lanes 1..28 (FS_OUT columns). At sweep row c the
 // warp receives E2 of row c+3 and U2*_B of row c+2, forms B2 and E3 of row c+2, B^{n+1} of row c+1
 // and writes B^{n+1} and the CFL speed of row c. x neighbours come from shuffles.
+//
+// Bound by memory: 70 bytes a zone. A warp's rows come through a shared-memory ring filled by cp.async,
+// three rows ahead; group g holds E2 of row g, U2*_B of row g-1 and the hydro of row g-3, which are all
+// used at sweep row c = g-3. (With one row ahead in registers a warp spent most of its time waiting.)
 #pragma once
 
 #include "mhd_kernels.cuh"
@@ -15,7 +19,11 @@
 namespace mhd {
 
 constexpr int FS_OUT = 28;
-constexpr int FS_WARPS = 8;
+constexpr int FS_WARPS = 1;   // warps (independent strip segments) per block
+constexpr int FS_RING = 4;    // groups of rows per warp (power of two)
+constexpr int FS_SLOT = 7 * 32;
+constexpr size_t kFinSmemBytes = (size_t)FS_WARPS * FS_RING * FS_SLOT * sizeof(double);
+constexpr int kFinMinBlocks = 24 / FS_WARPS;  // resident warps per SM: at most 80 registers
 constexpr int FS_PRE = 3;  // rows swept before the first output row
 
 // A finalize sweep reaches its grid through an accessor FA: acc(q) the accumulator planes (U2*),
@@ -43,7 +51,8 @@ struct FinParams {
 // The sweep of one warp over rows [r0, r1) of column strip sx of one grid.
 template <class FA>
 __device__ __forceinline__ void finalize_sweep_warp(const FA& f, const StepCoeffs* __restrict__ C,
-                                                    DeviceStatus* st, int sx, int r0, int r1) {
+                                                    DeviceStatus* st, int sx, int r0, int r1,
+                                                    double* ring) {
     const int lane = threadIdx.x & 31;
     const int nx = f.nx();  // setup only: the loop reads the grid through f
     const int c0 = sx * FS_OUT;
@@ -59,33 +68,41 @@ __device__ __forceinline__ void finalize_sweep_warp(const FA& f, const StepCoeff
     auto sup = [](double v) { return __shfl_up_sync(0xffffffffu, v, 1); };
 
     const int cstart = r0 - FS_PRE;
-    // pipelines
-    double x_cur = __ldg(&f.x()[rowp(cstart + 2) + iw]);  // E2 row c+2
-    double x_in = __ldg(&f.x()[rowp(cstart + 3) + iw]);   // E2 row c+3 (arriving)
-    double b0x_in = f.acc(4)[rowp(cstart + 2) + iw];      // U2*_B row c+2 (arriving)
-    double b0y_in = f.acc(5)[rowp(cstart + 2) + iw];
+    auto slot = [&](int g) { return ring + ((g - cstart) & (FS_RING - 1)) * FS_SLOT + lane; };
+    auto issue = [&](int g) {
+        if (g < r1 + 3) {
+            double* sl = slot(g);
+            cp_async8(&sl[0], &f.x()[rowp(g) + iw]);
+            const size_t rf = rowp(g - 1) + iw;
+            cp_async8(&sl[32], &f.acc(4)[rf]);
+            cp_async8(&sl[64], &f.acc(5)[rf]);
+            if (g - 3 >= r0) {
+                const size_t rh = (size_t)(g - 3) * f.nx() + iw;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) cp_async8(&sl[96 + 32 * q], &f.acc(q)[rh]);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int g = 2; g < 2 + FS_RING; ++g) issue(cstart + g);  // (the first holds E2 of row cstart + 2)
+    cp_async_wait<FS_RING - 1>();
+    double xb = slot(cstart + 2)[0];                       // E2 row c+2
     double b0x[2] = {0.0, 0.0}, b0y[2] = {0.0, 0.0};       // U2*_B rows c, c+1
     double bx2_prev = 0.0;                                 // B2_x row c+1
     double e3_prev = 0.0;                                  // E3 row c+1
     double bnx_prev = 0.0, bny_prev = 0.0;                 // B^{n+1} row c
-    double h_cur[4] = {0.0, 0.0, 0.0, 0.0};                // U2* hydro of row c (prefetched)
     double vmax = 0.0;
     bool bad = false;
 
     for (int c = cstart; c < r1; ++c) {
-        const double xa = x_in, xb = x_cur;  // rows c+3, c+2
-        const double ux = b0x_in, uy = b0y_in;  // U2*_B row c+2
-        // issue the next row's loads
-        x_cur = xa;
-        x_in = __ldg(&f.x()[rowp(c + 4) + iw]);
-        b0x_in = f.acc(4)[rowp(c + 3) + iw];
-        b0y_in = f.acc(5)[rowp(c + 3) + iw];
-        double h_nx[4] = {0.0, 0.0, 0.0, 0.0};
-        if (out_lane && c + 1 >= r0 && c + 1 < r1) {
-            const size_t g = (size_t)(c + 1) * f.nx() + i;
+        cp_async_wait<FS_RING - 2>();  // group c+3 has landed
+        const double* sl = slot(c + 3);
+        const double xa = sl[0], ux = sl[32], uy = sl[64];  // E2 row c+3, U2*_B row c+2
+        double h_cur[4];                                    // U2* hydro of row c
 #pragma unroll
-            for (int q = 0; q < 4; ++q) h_nx[q] = f.acc(q)[g];
-        }
+        for (int q = 0; q < 4; ++q) h_cur[q] = sl[96 + 32 * q];
+        issue(c + 2 + FS_RING);  // into group c+2's slot
         // B2 of row c+2 (x neighbour of E2 from the next lane)
         const double bx2 = ux + (-(xa - xb) * idy) * cg;
         const double by2 = uy + ((sdn(xb) - xb) * idx) * cg;
@@ -118,9 +135,9 @@ __device__ __forceinline__ void finalize_sweep_warp(const FA& f, const StepCoeff
         e3_prev = e3;
         bnx_prev = bnx;
         bny_prev = bny;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) h_cur[q] = h_nx[q];
+        xb = xa;
     }
+    cp_async_wait<0>();  // leave no copy in flight into the ring
     for (int o = 16; o > 0; o >>= 1) vmax = smax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     const bool any_bad = __any_sync(0xffffffffu, bad);
     if (lane == 0) {
@@ -129,16 +146,22 @@ __device__ __forceinline__ void finalize_sweep_warp(const FA& f, const StepCoeff
     }
 }
 
-static __global__ void __launch_bounds__(32 * FS_WARPS)
+static __global__ void __launch_bounds__(32 * FS_WARPS, kFinMinBlocks)
 k_finalize_sweep(Domain D, const StepCoeffs* __restrict__ C, Planes acc,
                  const double* __restrict__ xsolve, double* __restrict__ bx_out,
                  double* __restrict__ by_out, DeviceStatus* st, SweepGeom G) {
+#if defined(__CUDA_ARCH__)
+    extern __shared__ __align__(16) double fs_ring_mem[];
+#else
+    static double fs_ring_mem[FS_WARPS * FS_RING * FS_SLOT];  // host compilation: one copy
+#endif
     const int w = blockIdx.x * FS_WARPS + (threadIdx.x >> 5);
     if (w >= G.nwarps) return;
     const int sx = w % G.strips_x, sy = w / G.strips_x;
     const int r0 = sy * G.seg_h;
     const FinParams f{acc, xsolve, bx_out, by_out, D};
-    finalize_sweep_warp(f, C, st, sx, r0, min(r0 + G.seg_h, D.ny));
+    finalize_sweep_warp(f, C, st, sx, r0, min(r0 + G.seg_h, D.ny),
+                        fs_ring_mem + (size_t)(threadIdx.x >> 5) * FS_RING * FS_SLOT);
 }
 
 }  // namespace mhd

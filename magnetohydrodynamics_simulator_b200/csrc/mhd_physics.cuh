@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 #include <math.h>
+#include <string.h>
 
 namespace mhd {
 
@@ -26,14 +27,76 @@ struct Flux {
     double rho, mx, my, E, bt;  // bt: the tangential induction flux (F^By in x, F^Bx in y)
 };
 
+// Reciprocal and square root as straight-line code: the hardware's approximation (relative error below
+// 2^-19; PTX rcp/rsqrt.approx.ftz.f64) and one third-order step (Householder 1970) for 1/a, one
+// Goldschmidt step and one residual correction (Markstein 1990) for sqrt(a). Largest error found against
+// the correctly rounded results, over 1.5e8 arguments of 2^-300 .. 2^300: 0.51 and 0.52 ulp. Their
+// arguments are normal numbers, positive for the root (0, infinities and subnormals give NaN). The library's
+// division and root branch to a slow path, and each such branch ends a basic block: with the eight roots and
+// seven reciprocals of a cell's two faces inline, both faces' arithmetic interleaves.
+__device__ __forceinline__ double rcp_nr(double a) {
+#if defined(__CUDA_ARCH__)
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double e = fma(-a, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+#else
+    return 1.0 / a;
+#endif
+}
+__device__ __forceinline__ double sqrt_nr(double a) {
+#if defined(__CUDA_ARCH__)
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double g = a * y, h = 0.5 * y;
+    const double g1 = fma(g, fma(-g, h, 0.5), g);
+    return fma(fma(-g1, g1, a), h, g1);
+#else
+    return sqrt(a);
+#endif
+}
+
+// X * rsqrt(X * r) = sqrt(X / r) for X, r > 0: one third-order step on the reciprocal root instead of a
+// reciprocal and a root.
+__device__ __forceinline__ double sqrt_quotient(double X, double r) {
+#if defined(__CUDA_ARCH__)
+    const double z = X * r;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(z));
+    const double e = fma(-(z * y), y, 1.0);
+    return X * fma(y * e, fma(0.375, e, 0.5), y);
+#else
+    return sqrt(X / r);
+#endif
+}
+
+// High word of a double, for tests of sign and magnitude by integer instructions.
+__device__ __forceinline__ int high_word(double v) {
+#if defined(__CUDA_ARCH__)
+    return __double2hiint(v);
+#else
+    long long b;
+    memcpy(&b, &v, sizeof(b));
+    return (int)(b >> 32);
+#endif
+}
+
 // std::min / std::max semantics (b < a ? b : a), not fmin/fmax.
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 
-// MUSCL.hpp:11-17
+// MUSCL.hpp:11-17. The test a * b > 0 by the sign bits: an integer instruction for a product and a
+// comparison of the FP64 pipe. (Where it differs -- a zero, a product that underflows -- the smaller operand
+// is below 1e-154; a NaN operand gives NaN or the other operand.)
 __device__ __forceinline__ double minmod(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    const double s = (fabs(a) < fabs(b)) ? a : b;
+    // (the high word decides: cleared, what is left of s is below 1e-313)
+    return __hiloint2double((__double2hiint(a) ^ __double2hiint(b)) >= 0 ? __double2hiint(s) : 0, __double2loint(s));
+#else
     if (a * b > 0.0) return (fabs(a) < fabs(b)) ? a : b;
     return 0.0;
+#endif
 }
 
 // MUSCL.hpp:26-47, lower (c - s/2) face value of a cell from (left, centre, right)
@@ -52,7 +115,7 @@ __device__ __forceinline__ double primitives(double& rho, double mx, double my, 
                                              double bxc, double byc, double& vx, double& vy) {
     // one reciprocal instead of two divisions (<= 1 ulp from m/rho; the reference's fast-math
     // build is free to do the same)
-    const double ir = 1.0 / rho;
+    const double ir = rcp_nr(rho);
     vx = mx * ir;
     vy = my * ir;
     if (rho < kRhoFloor) rho = kRhoFloor;
@@ -64,16 +127,17 @@ __device__ __forceinline__ double primitives(double& rho, double mx, double my, 
     return p;
 }
 
-// HLL.hpp:107-122 fast magnetosonic speed
+// HLL.hpp:107-122 fast magnetosonic speed, c^2 = (s + sqrt(s^2 - 4 a^2 n^2)) / 2 with s = (gamma p + B^2) / rho,
+// a^2 = gamma p / rho, n^2 = Bn^2 / rho. All terms share 1 / rho, so it is taken once, under the root:
+// c = sqrt(X / rho), X = S + sqrt(S^2 - gamma p Bn^2), S = (gamma p + B^2) / 2.
 __device__ __forceinline__ double fast_speed(const Prim& w, double bn) {
     const double b2 = w.bx * w.bx + w.by * w.by;
-    const double ir = 1.0 / w.rho;  // one reciprocal for the three quotients by rho
-    const double a2 = kGammaGas * w.p * ir;
-    const double t2 = b2 * ir;
-    const double n2 = bn * bn * ir;
-    const double sum = t2 + a2;
-    const double term = sum * sum - 4.0 * a2 * n2;
-    return sqrt(0.5 * (sum + sqrt(term > 0.0 ? term : 0.0)));
+    const double gp = kGammaGas * w.p;
+    const double S = 0.5 * (gp + b2);
+    const double D = fma(S, S, -(gp * (bn * bn)));
+    const double root = sqrt_nr(D);
+    // D <= 0 up to rounding, or below 2^-960, counts as 0 (S > 0: the pressure is floored)
+    return sqrt_quotient(S + (high_word(D) > 0x03f00000 ? root : 0.0), w.rho);
 }
 
 // HLL.hpp:61-104 physical flux normal to direction DIR (0 = x, 1 = y), together with the
@@ -111,18 +175,15 @@ __device__ __forceinline__ Flux conserved(const Prim& w) {
     U.my = w.rho * w.vy;
     const double v2 = w.vx * w.vx + w.vy * w.vy;
     const double b2 = w.bx * w.bx + w.by * w.by;
-    U.E = w.p * kInvGm1 + 0.5 * w.rho * v2 + 0.5 * b2;
+    U.E = w.p * kInvGm1 + 0.5 * (w.rho * v2 + b2);  // as phys_flux forms it: one value for both
     U.bt = (DIR == 0) ? w.by : w.bx;
     return U;
 }
 
-// HLL.hpp:126-172 (DIR = 0) and :177-218 (DIR = 1). L is the lower/left state. SELECT: form the
-// HLL average for every face and select the case afterwards instead of returning early (the same
-// values; straight-line code that schedules better where registers allow it, measured on B200:
-// stage 1 1.030 -> 1.010 ms at 4096^2; stage 2 uses it once its carried values live in shared
-// memory; in the batch's stage 2 it fits without spills too but gains nothing, 6.97-6.99 against
-// 6.98 ms per batched step, so the batch keeps the branches).
-template <int DIR, bool SELECT = false>
+// HLL.hpp:126-172 (DIR = 0) and :177-218 (DIR = 1). L is the lower/left state. The reference takes F_L where
+// sL >= 0, F_R where sR <= 0 and the average between; with sL and sR clamped to the two sides of 0 the
+// average's own weights give those cases, to rounding: straight-line code without selects per component.
+template <int DIR>
 __device__ __forceinline__ Flux hll(const Prim& L, const Prim& R) {
     const Flux FL = phys_flux<DIR>(L);
     const Flux FR = phys_flux<DIR>(R);
@@ -130,41 +191,20 @@ __device__ __forceinline__ Flux hll(const Prim& L, const Prim& R) {
     const double cR = fast_speed(R, DIR == 0 ? R.bx : R.by);
     const double vL = DIR == 0 ? L.vx : L.vy;
     const double vR = DIR == 0 ? R.vx : R.vy;
-    const double sL = smin(vL - cL, vR - cR);
-    const double sR = smax(vL + cL, vR + cR);
-    if constexpr (SELECT) {
-        // sR = sL only where the selection takes F_L or F_R
-        const Flux UL = conserved<DIR>(L);
-        const Flux UR = conserved<DIR>(R);
-        const double inv = 1.0 / (sR - sL);
-        const double sLR = sL * sR;
-        const bool left = sL >= 0, right = !left && sR <= 0;
-        auto pick = [&](double fl, double fr, double ul, double ur) {
-            const double avg = (sR * fl - sL * fr + sLR * (ur - ul)) * inv;
-            return left ? fl : (right ? fr : avg);
-        };
-        Flux F;
-        F.rho = pick(FL.rho, FR.rho, UL.rho, UR.rho);
-        F.mx = pick(FL.mx, FR.mx, UL.mx, UR.mx);
-        F.my = pick(FL.my, FR.my, UL.my, UR.my);
-        F.E = pick(FL.E, FR.E, UL.E, UR.E);
-        F.bt = pick(FL.bt, FR.bt, UL.bt, UR.bt);
-        return F;
-    } else {
-        if (sL >= 0) return FL;
-        if (sR <= 0) return FR;
-        const Flux UL = conserved<DIR>(L);
-        const Flux UR = conserved<DIR>(R);
-        const double inv = 1.0 / (sR - sL);
-        const double sLR = sL * sR;
-        Flux F;
-        F.rho = (sR * FL.rho - sL * FR.rho + sLR * (UR.rho - UL.rho)) * inv;
-        F.mx = (sR * FL.mx - sL * FR.mx + sLR * (UR.mx - UL.mx)) * inv;
-        F.my = (sR * FL.my - sL * FR.my + sLR * (UR.my - UL.my)) * inv;
-        F.E = (sR * FL.E - sL * FR.E + sLR * (UR.E - UL.E)) * inv;
-        F.bt = (sR * FL.bt - sL * FR.bt + sLR * (UR.bt - UL.bt)) * inv;
-        return F;
-    }
+    const double mn = smin(vL - cL, vR - cR), mx = smax(vL + cL, vR + cR);
+    const double sL = high_word(mn) < 0 ? mn : 0.0, sR = high_word(mx) < 0 ? 0.0 : mx;
+    const Flux UL = conserved<DIR>(L);
+    const Flux UR = conserved<DIR>(R);
+    const double inv = rcp_nr(sR - sL);
+    const double a = sR * inv, b = sL * inv, c = sR * b;
+    auto avg = [&](double fl, double fr, double ul, double ur) { return fma(c, ur - ul, fma(a, fl, -(b * fr))); };
+    Flux F;
+    F.rho = avg(FL.rho, FR.rho, UL.rho, UR.rho);
+    F.mx = avg(FL.mx, FR.mx, UL.mx, UR.mx);
+    F.my = avg(FL.my, FR.my, UL.my, UR.my);
+    F.E = avg(FL.E, FR.E, UL.E, UR.E);
+    F.bt = avg(FL.bt, FR.bt, UL.bt, UR.bt);
+    return F;
 }
 
 // solvers.hpp:326,333 corner-velocity test. GCC resolves the unqualified abs(double) there to
@@ -173,7 +213,8 @@ __device__ __forceinline__ Flux hll(const Prim& L, const Prim& R) {
 // |v| < 1e-12 test, for physics studies.
 __device__ __forceinline__ bool ct_average(double v, int mode) {
     if (mode == 1) return fabs(v) < 1e-12;
-    return !(fabs(v) >= 1.0 && fabs(v) < 2147483648.0);
+    const unsigned a = (unsigned)high_word(v) & 0x7fffffffu;  // |v| >= 1 and |v| < 2^31 by the exponent
+    return !(a >= 0x3ff00000u && a < 0x41e00000u);
 }
 
 // solvers.hpp:314-340 corner electric field from the four face fluxes and the corner velocity.
@@ -181,9 +222,9 @@ __device__ __forceinline__ double corner_ez(double eN, double eS, double eE, dou
                                             double vyc, int mode) {
     double ezy, ezx;
     if (ct_average(vyc, mode)) ezy = 0.5 * (eS + eN);
-    else ezy = (vyc > 0.0) ? eS : eN;
+    else ezy = (high_word(vyc) > 0) ? eS : eN;
     if (ct_average(vxc, mode)) ezx = 0.5 * (eE + eW);
-    else ezx = (vxc > 0.0) ? eW : eE;
+    else ezx = (high_word(vxc) > 0) ? eW : eE;
     return 0.5 * (ezx + ezy);
 }
 
@@ -192,10 +233,12 @@ __device__ __forceinline__ double cfl_speed(double rho_f, double vx, double vy, 
                                             double bxc, double byc) {
     const double r = smax(rho_f, 1e-8);
     const double pr = smax(p, 1e-8);
-    const double ir = 1.0 / r;
+    const double ir = rcp_nr(r);
     const double a2 = kGammaGas * pr * ir;
     const double b2 = (bxc * bxc + byc * byc) * ir;
-    return sqrt(a2 + b2) + sqrt(vx * vx + vy * vy);
+    const double v2 = vx * vx + vy * vy;
+    const double v = sqrt_nr(v2);
+    return sqrt_nr(a2 + b2) + (v2 > 1e-290 ? v : 0.0);
 }
 
 }  // namespace mhd

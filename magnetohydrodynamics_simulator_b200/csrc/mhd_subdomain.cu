@@ -948,7 +948,7 @@ mhd_status mhd_sub_create(const mhd_params* p, void* stream, mhd_subdomain** out
     }
     {
         int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finalize_sweep, 32 * FS_WARPS, kFinSmemBytes) !=
                 cudaSuccess || occ < 1)
             return fail(MHD_ERR_CUDA);
         const long long resident = (long long)occ * s->num_sms * FS_WARPS;
@@ -1256,7 +1256,7 @@ mhd_status mhd_sub_finalize(mhd_subdomain* s) {
     if (st != MHD_OK) return st;
     Planes A;
     for (int k = 0; k < 6; ++k) A.f[k] = s->A[k];
-    k_finalize_sweep<<<s->fn_blocks, 32 * FS_WARPS, 0, s->stream>>>(s->ext, s->coeffs, A, s->V.x, s->S[4],
+    k_finalize_sweep<<<s->fn_blocks, 32 * FS_WARPS, kFinSmemBytes, s->stream>>>(s->ext, s->coeffs, A, s->V.x, s->S[4],
                                                                     s->S[5], s->scratch_status, s->fg);
     MHD_TRY(cudaGetLastError());
     // the accumulator's hydro planes hold U^{n+1}: they become the state's (pointer swap)

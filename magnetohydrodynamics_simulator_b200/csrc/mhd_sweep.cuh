@@ -28,20 +28,25 @@
 namespace mhd {
 
 constexpr int SW_OUT = 28;       // output columns per warp
-// The input rows are kept in a per-warp shared-memory ring filled by cp.async, not in registers.
-// Slot layout: rho, mx, my, E, bxf, byf of the warp's 32 columns at q*32 + lane, lane 31's
-// right-hand neighbour bxf(i+1) at 192; stage 2 adds E1 at SW_E1 + lane and lane 31's right-hand
-// E1 at SW_E1 + 32.
-constexpr int SW_RING = 8;       // row slots per warp (power of two): rows c-1 .. c+6
-constexpr int SW_E1 = 196;       // offset of E1 in a stage-2 slot
-constexpr int SW_SLOT = 230;     // doubles per slot (1840 bytes, 16-byte multiple)
+// The input rows are kept in per-warp shared-memory rings filled by cp.async, not in registers:
+//   hydro  rho, mx, my, E of a row at q*32 + lane. Stage 1 adds row c's to its outputs (8 rows: c .. c+7),
+//          stage 2 only forms the primitives of row c+2 from them (4 rows: c+2 .. c+5);
+//   faces  bxf, byf, and lane 31's right-hand neighbour bxf(i+1) at SW_FR: 8 rows, c-1 .. c+6;
+//   E1     stage 2's corner field, lane 31's right-hand neighbour at 32: 4 rows, c+3 .. c+6.
+// Every ring has a power of two of rows; 16 warps' rings fit an SM.
+constexpr int SW_FROWS = 8;      // face rows
+constexpr int SW_FSLOT = 66;     // doubles of a face row
+constexpr int SW_FR = 64;
+constexpr int SW_EROWS = 4;      // E1 rows (stage 2)
+constexpr int SW_ESLOT = 34;
+constexpr int sw_hrows(int mode) { return mode == 1 ? 8 : 4; }  // hydro rows
 // Stage 2 keeps the values it carries from row to row -- the y slopes and the y-face fluxes of the
-// previous row, 10 per lane -- in shared memory after its ring, not in registers. The registers it
-// frees let stage 2 evaluate HLL branch-free as stage 1 does (measured on B200 at 4096^2: stage 2
-// 1.001 -> 0.954 ms; stage 1, whose carried values fit its registers, is 1.7% slower this way).
+// previous row, 10 per lane -- in shared memory after its rings, not in registers.
 constexpr int SW_CARRY = 10 * 32;
-// doubles of shared memory per warp of an explicit-stage kernel
-constexpr int sweep_warp_doubles(int mode) { return SW_RING * SW_SLOT + (mode == 2 ? SW_CARRY : 0); }
+// doubles of shared memory per warp of an explicit-stage kernel: 12.4 and 12.0 KB
+constexpr int sweep_warp_doubles(int mode) {
+    return sw_hrows(mode) * 128 + SW_FROWS * SW_FSLOT + (mode == 2 ? SW_EROWS * SW_ESLOT + SW_CARRY : 0);
+}
 // One warp (an independent strip segment) per block: blocks retire warp by warp, so the tail of
 // a launch and the persistent batch kernels balance at warp granularity (measured on B200 against
 // 4-warp blocks at the same registers: stage 1 1.29 -> 1.25 ms, stage 2 1.24 -> 1.15 ms at 4096^2).
@@ -49,7 +54,9 @@ constexpr int sweep_warp_doubles(int mode) { return SW_RING * SW_SLOT + (mode ==
 #define MHD_SW_WARPS 1
 #endif
 constexpr int SW_WARPS = MHD_SW_WARPS;  // warps (independent strips) per block
-constexpr int SW_PRE = 5;        // rows swept before the first output row of a strip
+// Rows swept before the first output row: the windows take PRIM from row r0 - 2 on (and stage 2 one more row
+// to turn the first faces into B1); the faces, the costly part, start one row before the first output.
+constexpr int sw_pre(int mode) { return mode == 1 ? 4 : 5; }
 
 __device__ __forceinline__ double shup(double v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
 __device__ __forceinline__ double shdn(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
@@ -134,9 +141,14 @@ struct RecPlanes {
     __device__ __forceinline__ int ct_mode() const { return vload(&rec->D.ct_mode); }
 };
 
+template <bool V>
+struct SwTag {
+    static constexpr bool value = V;
+};
+
 // The sweep of one warp over rows [r0, r1) of column strip sx of one grid.
 template <int MODE, class PL, bool kYReuse = (MODE == 1) ? MHD_SWEEP_YREUSE_1 : MHD_SWEEP_YREUSE_2,
-          bool kXReuse = (MODE == 1) ? MHD_SWEEP_XREUSE_1 : MHD_SWEEP_XREUSE_2, bool kSelect = true>
+          bool kXReuse = (MODE == 1) ? MHD_SWEEP_XREUSE_1 : MHD_SWEEP_XREUSE_2>
 __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ C, const PL& pl,
                                                  int sx, int r0, int r1, double* ring) {
     const int lane = threadIdx.x & 31;
@@ -165,7 +177,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
     // y slopes of row c (when carried) and the y-face flux of row c-1: registers in stage 1,
     // shared memory after the ring in stage 2
     double Sy_r[5], fy_r[5];
-    double* const carry = ring + SW_RING * SW_SLOT;
+    double* const carry = ring + sw_hrows(2) * 128 + SW_FROWS * SW_FSLOT + SW_EROWS * SW_ESLOT;
     auto Sy = [&](int k) -> double& {
         if constexpr (MODE == 2) return carry[(5 + k) * 32 + lane];
         else return Sy_r[k];
@@ -182,51 +194,69 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
 #pragma unroll
     for (int k = 0; k < 5; ++k) { Sy(k) = 0.0; fy_prev(k) = 0.0; }
 
-    const int cstart = r0 - SW_PRE;
-    // The input rows live in the ring: sweep row r sits in slot (r - cstart + 1) % SW_RING; it is
-    // copied while the warp works on row r - 7 and read up to row r + 1. Stage 2 also copies E1 and
-    // turns the row's faces into B1 when the row arrives (B1 is what every later read of the row
-    // needs).
-    auto slot = [&](int r) -> double* {
-        return ring + (unsigned)((r - cstart + 1) & (SW_RING - 1)) * SW_SLOT;
+    const int cstart = r0 - sw_pre(MODE);
+    // Sweep row r sits in slot (r - cstart) % rows of its ring. Group r, issued at the end of row r - 7,
+    // copies faces and E1 of row r and the hydro of row r (stage 1) or r - 1 (stage 2): each into the slot
+    // of a row no longer read. Stage 2 turns a row's faces into B1 when the row arrives (B1 is what every
+    // later read of the row needs).
+    constexpr int HR = sw_hrows(MODE);
+    auto hyd = [&](int r) -> double* { return ring + ((r - cstart) & (HR - 1)) * 128; };
+    auto fac = [&](int r) -> double* { return ring + HR * 128 + ((r - cstart) & (SW_FROWS - 1)) * SW_FSLOT; };
+    auto e1row = [&](int r) -> double* {
+        return ring + HR * 128 + SW_FROWS * SW_FSLOT + ((r - cstart) & (SW_EROWS - 1)) * SW_ESLOT;
     };
     auto issue_row = [&](int r) {
         if (r <= r1 + (MODE == 1 ? 3 : 4)) {
-            double* sl = slot(r);
             const size_t rp = rowp(r);
-#pragma unroll
-            for (int q = 0; q < 6; ++q) cp_async8(&sl[q * 32 + lane], &pl.in(q)[rp + iw]);
-            if (lane == 31) cp_async8(&sl[192], &pl.in(4)[rp + iw_r]);
+            double* f = fac(r);
+            cp_async8(&f[lane], &pl.in(4)[rp + iw]);
+            cp_async8(&f[32 + lane], &pl.in(5)[rp + iw]);
+            if (lane == 31) cp_async8(&f[SW_FR], &pl.in(4)[rp + iw_r]);
             if constexpr (MODE == 2) {
-                cp_async8(&sl[SW_E1 + lane], &pl.x()[rp + iw]);
-                if (lane == 31) cp_async8(&sl[SW_E1 + 32], &pl.x()[rp + iw_r]);
+                // (the first rows of the short rings are not used: their slots belong to later rows)
+                if (r >= cstart + 3) {
+                    double* e = e1row(r);
+                    cp_async8(&e[lane], &pl.x()[rp + iw]);
+                    if (lane == 31) cp_async8(&e[32], &pl.x()[rp + iw_r]);
+                    const size_t rh = rowp(r - 1);
+                    double* h = hyd(r - 1);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) cp_async8(&h[q * 32 + lane], &pl.in(q)[rh + iw]);
+                }
+            } else {
+                double* h = hyd(r);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) cp_async8(&h[q * 32 + lane], &pl.in(q)[rp + iw]);
             }
         }
         cp_async_commit();
     };
 #pragma unroll
-    for (int r = 0; r < SW_RING; ++r) issue_row(cstart - 1 + r);
+    for (int r = 0; r < SW_FROWS; ++r) issue_row(cstart - 1 + r);
 
-    for (int c = cstart; c <= r1; ++c) {
-        if constexpr (MODE == 1) cp_async_wait<SW_RING - 5>();  // rows up to c+3 have landed
-        else cp_async_wait<SW_RING - 6>();                       // rows up to c+4 have landed
+    // One sweep row; kFaces: with the faces, the corner and the outputs (from row r0 - 1 on).
+    auto row = [&](int c, auto faces) {
+        constexpr bool kFaces = decltype(faces)::value;
+        if constexpr (MODE == 1) cp_async_wait<3>();  // rows up to c+3 have landed
+        else cp_async_wait<2>();                       // rows up to c+4 have landed
         // stage 2: the accumulator values this row's outputs add to (hydro row c, faces row c-1),
         // loaded here and used at the end of the row
         double accH[4] = {0.0, 0.0, 0.0, 0.0}, accB[2] = {0.0, 0.0};
         if constexpr (MODE == 2) {
             // B1 = U1*_B + dt*g*(rate of E1) of row c+3 (solvers.hpp:484-485, 528-529), written
             // over the row's faces in the ring (lane 31 also converts its right-hand bxf)
-            double* s3 = slot(c + 3);
-            const double* s4 = slot(c + 4);
-            const double ax0 = s3[SW_E1 + lane], ax1 = s4[SW_E1 + lane];
+            double* f3 = fac(c + 3);
+            const double* e3 = e1row(c + 3);
+            const double* e4 = e1row(c + 4);
+            const double ax0 = e3[lane], ax1 = e4[lane];
             double axr = shdn(ax0, 1);
-            if (lane == 31) axr = s3[SW_E1 + 32];
+            if (lane == 31) axr = e3[32];
             const double rbx = -(ax1 - ax0) * idy;
             const double rby = (axr - ax0) * idx;
-            s3[4 * 32 + lane] = s3[4 * 32 + lane] + rbx * cg;
-            s3[5 * 32 + lane] = s3[5 * 32 + lane] + rby * cg;
-            if (lane == 31) s3[192] = s3[192] + (-(s4[SW_E1 + 32] - s3[SW_E1 + 32]) * idy) * cg;
-            if (out_lane) {
+            f3[lane] = f3[lane] + rbx * cg;
+            f3[32 + lane] = f3[32 + lane] + rby * cg;
+            if (lane == 31) f3[SW_FR] = f3[SW_FR] + (-(e4[32] - e3[32]) * idy) * cg;
+            if (kFaces && out_lane) {
                 if (c >= r0 && c < r1) {
                     const size_t g = (size_t)c * pl.nx() + i;
 #pragma unroll
@@ -243,15 +273,16 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         //      and c+3; bxf one column to the right from the next lane (lane 31: its own copy)
         double nrho, nvx, nvy, np, nbxc, nbyc;
         {
-            const double* s2 = slot(c + 2);
-            const double bxf2 = s2[4 * 32 + lane];
+            const double* f2 = fac(c + 2);
+            const double* h2 = hyd(c + 2) + lane;
+            const double bxf2 = f2[lane];
             double bxr2 = shdn(bxf2, 1);
-            if (lane == 31) bxr2 = s2[192];
+            if (lane == 31) bxr2 = f2[SW_FR];
             nbxc = (bxf2 + bxr2) / 2.0;
-            nbyc = (s2[5 * 32 + lane] + slot(c + 3)[5 * 32 + lane]) / 2.0;
-            double rho = s2[lane];
+            nbyc = (f2[32 + lane] + fac(c + 3)[32 + lane]) / 2.0;
+            double rho = h2[0];
             if (MODE == 2 && rho < kRhoFloor) rho = kRhoFloor;  // floored in place (solvers.hpp:522-523)
-            np = primitives(rho, s2[32 + lane], s2[64 + lane], s2[96 + lane], nbxc, nbyc, nvx, nvy);
+            np = primitives(rho, h2[32], h2[64], h2[96], nbxc, nbyc, nvx, nvy);
             nrho = rho;
         }
 #pragma unroll
@@ -264,6 +295,17 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         // window rows now: P*[0..3] = c-1 .. c+2, Pbyc[0..2] = c .. c+2; ring rows c-1 .. c+3
         //                  (stage 2: their faces hold B1)
 
+        if constexpr (!kFaces) {
+            if constexpr (kYReuse) {  // the slopes that the first face row takes over
+                Sy(0) = minmod(Prho[2] - Prho[1], Prho[3] - Prho[2]);
+                Sy(1) = minmod(Pvx[2] - Pvx[1], Pvx[3] - Pvx[2]);
+                Sy(2) = minmod(Pvy[2] - Pvy[1], Pvy[3] - Pvy[2]);
+                Sy(3) = minmod(Pp[2] - Pp[1], Pp[3] - Pp[2]);
+                Sy(4) = minmod(Pbxc[2] - Pbxc[1], Pbxc[3] - Pbxc[2]);
+            }
+            issue_row(c + 7);
+            return;
+        }
         // ---- YFACE: top face of (i, c); D = upper y-extrapolation of row c, U = lower of c+1
         //      (MUSCL.hpp:26-47). With kYReuse each row's limited slope is formed once, when the
         //      row is c+1, and carried to the next row for its upper extrapolation.
@@ -299,8 +341,8 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
                 Up.p = recon_lo(Pp[1], Pp[2], Pp[3]);
                 Up.bx = recon_lo(Pbxc[1], Pbxc[2], Pbxc[3]);
             }
-            Dn.by = Up.by = slot(c + 1)[5 * 32 + lane];  // byf of row c+1
-            fy = hll<1, kSelect>(Dn, Up);
+            Dn.by = Up.by = fac(c + 1)[32 + lane];  // byf of row c+1
+            fy = hll<1>(Dn, Up);
         }
         // ---- XFACE: right face of (i, c); L = upper x-extrapolation of column i, R = lower of
         //      i+1. With kXReuse every lane limits its own column's slope once and hands its lower
@@ -311,7 +353,8 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             Prim L, R;
             auto xrecon = [&](double q, double& hi, double& lo_right) {
                 if constexpr (kXReuse) {
-                    const double s = minmod(q - shup(q, 1), shdn(q, 1) - q);
+                    const double dl = q - shup(q, 1);
+                    const double s = minmod(dl, shdn(dl, 1));
                     hi = q + 0.5 * s;
                     lo_right = shdn(q - 0.5 * s, 1);
                 } else {
@@ -325,8 +368,8 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             xrecon(Pvy[1], L.vy, R.vy);
             xrecon(Pp[1], L.p, R.p);
             xrecon(Pbyc[0], L.by, R.by);
-            L.bx = R.bx = shdn(slot(c)[4 * 32 + lane], 1);  // bxf(i+1, c)
-            fx = hll<0, kSelect>(L, R);
+            L.bx = R.bx = shdn(fac(c)[lane], 1);  // bxf(i+1, c)
+            fx = hll<0>(L, R);
         }
         // ---- CORNER (i, c): eN = -Fx^By(i-1, c), eS = -Fx^By(i-1, c-1), eE = Fy^Bx(i, c-1),
         //      eW = Fy^Bx(i-1, c-1); corner velocity = mean of the 4 cells
@@ -342,9 +385,9 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         }
         double jz = 0.0;
         if (MODE == 2) {  // eta*J_z(B1) at corner (i, c) (solvers.hpp:450-461)
-            const double by1 = slot(c)[5 * 32 + lane];
+            const double by1 = fac(c)[32 + lane];
             const double dBy_dx = (by1 - shup(by1, 1)) * idx;
-            const double dBx_dy = (slot(c)[4 * 32 + lane] - slot(c - 1)[4 * 32 + lane]) * idy;
+            const double dBx_dy = (fac(c)[lane] - fac(c - 1)[lane]) * idy;
             jz = pl.eta() * (dBy_dx - dBx_dy);
         }
         // ---- hydro rates of row c
@@ -357,10 +400,10 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             if (out_lane && c >= r0 && c < r1) {
                 const size_t g = (size_t)c * pl.nx() + i;
                 if constexpr (MODE == 1) {
-                    const double* sc = slot(c);
+                    const double* hc = hyd(c) + lane;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const double u = sc[q * 32 + lane];
+                        const double u = hc[q * 32];
                         pl.a(q)[g] = u + f[q] * cA;                       // predictor
                         const double ua = (q == 0 && u < kRhoFloor) ? kRhoFloor : u;
                         pl.b(q)[g] = ua + f[q] * cB;                      // accumulator
@@ -383,8 +426,8 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             if (out_lane && c - 1 >= r0 && c - 1 < r1) {
                 const size_t g = (size_t)(c - 1) * pl.nx() + i;
                 if constexpr (MODE == 1) {
-                    const double* sp = slot(c - 1);
-                    const double ubx = sp[4 * 32 + lane], uby = sp[5 * 32 + lane];  // U^n faces, row c-1
+                    const double* fp = fac(c - 1);
+                    const double ubx = fp[lane], uby = fp[32 + lane];  // U^n faces, row c-1
                     pl.a(4)[g] = ubx + fbx * cA;
                     pl.a(5)[g] = uby + fby * cA;
                     pl.b(4)[g] = ubx + fbx * cB;
@@ -405,7 +448,9 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         ez_prev = ez;
         jz_prev = jz;
         issue_row(c + 7);  // into the slot of row c-1, no longer read
-    }
+    };
+    for (int c = cstart; c < r0 - 1; ++c) row(c, SwTag<false>{});
+    for (int c = r0 - 1; c <= r1; ++c) row(c, SwTag<true>{});
     cp_async_wait<0>();  // leave no copy in flight into the ring
 }
 
@@ -421,7 +466,7 @@ k_stage_sweep(Domain D, const StepCoeffs* __restrict__ C, CPlanes in,
 #if defined(__CUDA_ARCH__)
     extern __shared__ __align__(16) double sw_ring_mem[];
 #else
-    static double sw_ring_mem[SW_WARPS * (SW_RING * SW_SLOT + SW_CARRY)];  // host compilation: one copy
+    static double sw_ring_mem[SW_WARPS * (sweep_warp_doubles(1) + sweep_warp_doubles(2))];  // host compilation: one copy
 #endif
     double* const ring = sw_ring_mem + (size_t)(threadIdx.x >> 5) * sweep_warp_doubles(MODE);
     const int w = blockIdx.x * SW_WARPS + (threadIdx.x >> 5);
