@@ -155,8 +155,8 @@ mhd_status solve(mhd_adjoint* a, const double* bxf, const double* byf, double rh
     g.max_iters = a->prm.cg_max_iters > 0 ? a->prm.cg_max_iters : 2LL * (long long)a->n;
     g.tol = a->prm.cg_tol > 0 ? a->prm.cg_tol : 2.220446049250313e-16;
     g.timeout_s = a->prm.cg_timeout_s;
-    return mhd_host::launch_solve(g, a->geom, mhd_host::solve_t((a->dt * a->eta) * a->g, a->prm.dx, a->prm.dy), a->sync,
-                                  a->stream);
+    return mhd_host::launch_solve(g, a->geom, mhd_host::solve_t((a->dt * a->eta) * a->g, a->prm.dx, a->prm.dy), false,
+                                  a->sync, a->stream);
 }
 
 // One forward step from U into slot sl (U^{n+1} = (sl.A[0..3], sl.Bn)) with the corner fields of

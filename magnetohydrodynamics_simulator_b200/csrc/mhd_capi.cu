@@ -105,8 +105,8 @@ mhd_status launch_coeffs(mhd_context* c, double dt, int alpha_mode, double t_end
     return MHD_OK;
 }
 
-// t: the solve's t where the host knows it, else negative (mhd_host::launch_solve).
-mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int solve_index, double t,
+// t: the solve's t where the host knows it, else negative; field: a caller's field (mhd_host::launch_solve).
+mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int solve_index, double t, bool field,
                      long long* prods_out) {
     CgSweepArgs a{};
     a.D = c->dom;
@@ -125,7 +125,7 @@ mhd_status launch_cg(mhd_context* c, const double* bxf, const double* byf, int s
     a.max_iters = c->prm.cg_max_iters > 0 ? c->prm.cg_max_iters : 2LL * (long long)c->n;
     a.tol = c->prm.cg_tol > 0 ? c->prm.cg_tol : 2.220446049250313e-16;
     a.timeout_s = c->prm.cg_timeout_s;
-    return mhd_host::launch_solve(a, c->solve, t, c->sync, c->stream);
+    return mhd_host::launch_solve(a, c->solve, t, field, c->sync, c->stream);
 }
 
 // t of a step's solves for the given dt; negative for a CFL step, whose dt the device chooses. (A run's
@@ -173,14 +173,14 @@ mhd_status enqueue_step_body(mhd_context* c, double dt, long long* prods_out) {
         c->dom, c->coeffs, cplanes(c->S), nullptr, planes(c->T), planes(c->A), c->sg[0]);
     MHD_TRY(cudaGetLastError());
     MHD_MARK(c);
-    mhd_status s = launch_cg(c, c->T[4], c->T[5], 0, t, prods_out);
+    mhd_status s = launch_cg(c, c->T[4], c->T[5], 0, t, false, prods_out);
     if (s != MHD_OK) return s;
     MHD_MARK(c);
     k_stage_sweep<2><<<c->st_blocks[1], 32 * SW_WARPS, sweep_smem_bytes(2), c->stream>>>(
         c->dom, c->coeffs, cplanes(c->T), c->x, planes(c->T), planes(c->A), c->sg[1]);
     MHD_TRY(cudaGetLastError());
     MHD_MARK(c);
-    s = launch_cg(c, c->A[4], c->A[5], 1, t, prods_out);
+    s = launch_cg(c, c->A[4], c->A[5], 1, t, false, prods_out);
     if (s != MHD_OK) return s;
     MHD_MARK(c);
     k_finalize_sweep<<<c->fn_blocks, 32 * FS_WARPS, kFinSmemBytes, c->stream>>>(
@@ -765,7 +765,7 @@ mhd_status mhd_resistive_rate(mhd_context* c, int solve_implicitly, double alpha
     if (solve_implicitly) {
         k_set_alpha<<<1, 1, 0, c->stream>>>(c->coeffs, alpha);
         MHD_TRY(cudaGetLastError());
-        s = launch_cg(c, bxf, byf, 0, mhd_host::solve_t(alpha, c->prm.dx, c->prm.dy), nullptr);
+        s = launch_cg(c, bxf, byf, 0, mhd_host::solve_t(alpha, c->prm.dx, c->prm.dy), true, nullptr);
         if (s != MHD_OK) return s;
         k_corner_rates<<<blocks, 256, 0, c->stream>>>(c->dom, c->x, nullptr, nullptr, bx_rate, by_rate);
     } else {
@@ -1069,7 +1069,7 @@ extern "C" mhd_status mhd_resistive_rate_noalloc(const mhd_params* p, int solve_
     a.max_iters = p->cg_max_iters > 0 ? p->cg_max_iters : 2LL * (long long)n;
     a.tol = p->cg_tol > 0 ? p->cg_tol : 2.220446049250313e-16;
     a.timeout_s = p->cg_timeout_s > 0 ? p->cg_timeout_s : 30.0;
-    s = mhd_host::launch_solve(a, geom, mhd_host::solve_t(alpha, p->dx, p->dy), sync, stream);
+    s = mhd_host::launch_solve(a, geom, mhd_host::solve_t(alpha, p->dx, p->dy), true, sync, stream);
     if (s != MHD_OK) return s;
     k_corner_rates<<<blocks, 256, 0, stream>>>(D, x, nullptr, nullptr, bx_rate, by_rate);
     MHD_TRY(cudaGetLastError());

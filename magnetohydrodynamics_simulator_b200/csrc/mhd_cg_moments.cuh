@@ -39,15 +39,18 @@ constexpr int CM_NW = CM_NT / 32;
 constexpr int CM_RING = 8;  // prefetched rows per warp (power of two)
 constexpr int CM_MAXM = 9;  // levels of the longest pass 1
 constexpr int CM_NMU = 2 * CM_MAXM + 1;
-// Adjacent columns per lane (odd: conflict-free shared-memory reads), the halo lanes on each side of a pass
-// of M levels (M columns, whole lanes) and its output columns per warp. Measured at 4096^2, M = 7: 137 us;
-// two columns on 12 warps of 168 registers 156 us, on 16 warps of 128 registers the levels spill.
+// A pass works on C adjacent columns per lane: 3 (odd: conflict-free shared-memory reads), or 1 where the grid
+// has too few rows to keep the warps busy -- a row then takes a third of the instructions, which is what a
+// lone warp waits for, for twice the halo. Halo lanes on each side of a pass of M levels (M columns, whole
+// lanes) and output columns per warp. Measured at 4096^2, M = 7, C = 3: 137 us; two columns on 12 warps of
+// 168 registers 156 us, on 16 warps of 128 registers the levels spill.
 constexpr int CM_C = 3;
-__host__ __device__ constexpr int cm_halo_lanes(int M) { return (M + CM_C - 1) / CM_C; }
-__host__ __device__ constexpr int cm_out(int M) { return (32 - 2 * cm_halo_lanes(M)) * CM_C; }
-constexpr int CM_COLS = 32 * CM_C;
-constexpr int CM_SLOT = 2 * CM_COLS + 2;  // doubles of a ring slot: bx row, by row, by left of the first column
-constexpr int CM_WARP = CM_RING * CM_SLOT + CM_COLS;  // doubles of shared memory per warp: ring, an output row
+__host__ __device__ constexpr int cm_halo_lanes(int M, int C) { return (M + C - 1) / C; }
+__host__ __device__ constexpr int cm_out(int M, int C) { return (32 - 2 * cm_halo_lanes(M, C)) * C; }
+// Doubles of a ring slot (bx row, by row, by left of the first column) and of a warp's shared memory: ring,
+// then the staging of an output row.
+__host__ __device__ constexpr int cm_slot(int C) { return 2 * 32 * C + 2; }
+constexpr int CM_WARP = CM_RING * cm_slot(CM_C) + 32 * CM_C;
 constexpr size_t kCmSmemBytes = (size_t)CM_NW * CM_WARP * sizeof(double);
 static_assert(CG_RING * CG_SLOT <= CM_WARP, "the sweeps' rings fit the passes' shared memory");
 constexpr double kCmNoise = 5.7e-14;  // relative error allowed to the moment sums (256 eps)
@@ -63,15 +66,22 @@ __device__ __forceinline__ int cm_levels(double t) { return t < 1.2e-3 ? 5 : (t 
 struct CmSpan {
     int strips, seg_h, n;  // column strips, rows per segment, segments in all
 };
-// Split of the grid over `warps` warps: strips of `out` columns, row segments of equal height (at least
-// `min_rows`; short segments repeat 2 M halo rows each).
-__device__ __forceinline__ CmSpan cm_span(int nx, int ny, int out, int warps, int min_rows) {
+// Split of the grid over `warps` warps: strips of `out` columns, row segments of equal height (at least 4
+// rows: a segment repeats 2 M halo rows).
+__device__ __forceinline__ CmSpan cm_span(int nx, int ny, int out, int warps) {
     CmSpan s;
     s.strips = (nx + out - 1) / out;
     const int segs = max(1, warps / s.strips);
-    s.seg_h = max(min_rows, (ny + segs - 1) / segs);
+    s.seg_h = max(4, (ny + segs - 1) / segs);
     s.n = s.strips * ((ny + s.seg_h - 1) / s.seg_h);
     return s;
+}
+// Whether a pass of M levels is shorter with one column a lane: the rows of a warp's segment, weighed by what
+// a row takes a warp that has its scheduler nearly to itself (1700 cycles with three columns, 600 with one).
+__device__ __forceinline__ bool cm_narrow(int nx, int ny, int M, int warps) {
+    const CmSpan w = cm_span(nx, ny, cm_out(M, CM_C), warps), n = cm_span(nx, ny, cm_out(M, 1), warps);
+    const int rounds = (n.n + warps - 1) / warps;  // (a strip for every warp and more: very wide grids)
+    return rounds * (n.seg_h + 2 * M) * 6 < (w.seg_h + 2 * M) * 17;
 }
 
 struct CmGeom {
@@ -86,21 +96,22 @@ struct CmGeom {
 // A warp's stream of right-hand-side rows: cp.async into the ring, coalesced; each lane then reads
 // its C adjacent columns. Sweep row k holds grid row j0 + k (k = -1: only bx, the row below the
 // first). The caller runs next() once per row, in order.
+template <int C>
 struct CmRows {
     const CmGeom& g;
     double* ring;
     int lane, j0, last;  // grid row of sweep row 0, last sweep row
-    int col[CM_C], coll;    // wrapped columns this lane copies; the one left of the strip
+    int col[C], coll;    // wrapped columns this lane copies; the one left of the strip
 
     __device__ __forceinline__ CmRows(const CmGeom& g_, double* ring_, int c0, int j0_, int rows)
         : g(g_), ring(ring_), lane(threadIdx.x & 31), j0(j0_), last(rows - 1) {
 #pragma unroll
-        for (int q = 0; q < CM_C; ++q) col[q] = wrap(c0 + lane + 32 * q, g.nx);
+        for (int q = 0; q < C; ++q) col[q] = wrap(c0 + lane + 32 * q, g.nx);
         coll = wrap(c0 - 1, g.nx);
 #pragma unroll
         for (int k = -1; k < CM_RING - 2; ++k) issue(k);
     }
-    __device__ __forceinline__ double* slot(int k) const { return ring + ((k + 1) & (CM_RING - 1)) * CM_SLOT; }
+    __device__ __forceinline__ double* slot(int k) const { return ring + ((k + 1) & (CM_RING - 1)) * cm_slot(C); }
     __device__ __forceinline__ void issue(int k) const {
         if (k <= last) {
             const size_t rp = (size_t)wrap(j0 + k, g.ny) * g.nx;
@@ -108,27 +119,27 @@ struct CmRows {
             const double* px = g.bxf + rp;
             const double* py = g.byf + rp;
 #pragma unroll
-            for (int q = 0; q < CM_C; ++q) {
+            for (int q = 0; q < C; ++q) {
                 cp_async8(&s[lane + 32 * q], &px[col[q]]);
-                cp_async8(&s[CM_COLS + lane + 32 * q], &py[col[q]]);
+                cp_async8(&s[(32 * C) + lane + 32 * q], &py[col[q]]);
             }
-            if (lane == 0) cp_async8(&s[2 * CM_COLS], &py[coll]);
+            if (lane == 0) cp_async8(&s[2 * (32 * C)], &py[coll]);
         }
         cp_async_commit();
     }
     // b / scale of sweep row k at the lane's columns
-    __device__ __forceinline__ void next(int k, double (&b)[CM_C]) {
+    __device__ __forceinline__ void next(int k, double (&b)[C]) {
         cp_async_wait<CM_RING - 3>();  // row k has landed (row k + 1 may be in flight)
         __syncwarp();                  // ... for every lane, and every lane is done with row k - 1's slot
-        const double* s = slot(k) + lane * CM_C;
-        const double* sb = slot(k - 1) + lane * CM_C;  // the row below, still in its slot
-        double by[CM_C];
+        const double* s = slot(k) + lane * C;
+        const double* sb = slot(k - 1) + lane * C;  // the row below, still in its slot
+        double by[C];
 #pragma unroll
-        for (int c = 0; c < CM_C; ++c) by[c] = s[CM_COLS + c];
-        double byl = __shfl_up_sync(0xffffffffu, by[CM_C - 1], 1);
-        if (lane == 0) byl = s[2 * CM_COLS];
+        for (int c = 0; c < C; ++c) by[c] = s[(32 * C) + c];
+        double byl = __shfl_up_sync(0xffffffffu, by[C - 1], 1);
+        if (lane == 0) byl = s[2 * (32 * C)];
 #pragma unroll
-        for (int c = 0; c < CM_C; ++c) {
+        for (int c = 0; c < C; ++c) {
             b[c] = fma(g.ratio, sb[c] - s[c], by[c] - (c ? by[c - 1] : byl));
         }
         issue(k + CM_RING - 2);  // into row k - 2's slot
@@ -136,13 +147,14 @@ struct CmRows {
 };
 
 // D at one row: out = ctr - ax (left + right) - ay (below + above).
-__device__ __forceinline__ void cm_apply(const CmGeom& g, const double (&below)[CM_C], const double (&ctr)[CM_C],
-                                         const double (&above)[CM_C], double (&out)[CM_C]) {
-    const double l = __shfl_up_sync(0xffffffffu, ctr[CM_C - 1], 1);
+template <int C>
+__device__ __forceinline__ void cm_apply(const CmGeom& g, const double (&below)[C], const double (&ctr)[C],
+                                         const double (&above)[C], double (&out)[C]) {
+    const double l = __shfl_up_sync(0xffffffffu, ctr[C - 1], 1);
     const double r = __shfl_down_sync(0xffffffffu, ctr[0], 1);
 #pragma unroll
-    for (int c = 0; c < CM_C; ++c) {
-        const double lr = (c ? ctr[c - 1] : l) + (c < CM_C - 1 ? ctr[c + 1] : r);
+    for (int c = 0; c < C; ++c) {
+        const double lr = (c ? ctr[c - 1] : l) + (c < C - 1 ? ctr[c + 1] : r);
         out[c] = fma(-g.ay, below[c] + above[c], fma(-g.ax, lr, ctr[c]));
     }
 }
@@ -165,19 +177,19 @@ struct CmTag {
 // Pass 1 over rows [r0, r1) of strip sx: acc[2l] += w_l . w_l, acc[2l - 1] += w_l . w_{l-1}. FULL: every
 // column of the strip's output lanes counts (halo lanes' sums are dropped by the caller); else columns are
 // masked one by one.
-template <int M, bool FULL>
+template <int M, int C, bool FULL>
 __device__ __forceinline__ void cm_moments_segment(const CmGeom& g, int sx, int r0, int r1, double* smem,
                                                    double (&acc)[2 * M + 1]) {
-    constexpr int C = CM_C, LH = cm_halo_lanes(M);
+    constexpr int LH = cm_halo_lanes(M, C);
     const int lane = threadIdx.x & 31;
-    const int c0 = sx * cm_out(M) - LH * C;
+    const int c0 = sx * cm_out(M, C) - LH * C;
     const int h = r1 - r0;
     int own[C];  // all ones where the lane's column counts
 #pragma unroll
     for (int c = 0; c < C; ++c)
         own[c] = FULL || (lane >= LH && lane < 32 - LH && c0 + lane * C + c < g.nx) ? -1 : 0;
     const int rows = h + 2 * M;
-    CmRows in(g, smem, c0, r0 - M, rows);
+    CmRows<C> in(g, smem, c0, r0 - M, rows);
     // the two latest rows of w_0 .. w_{M-1}: S[k & 1] holds row k's, written over row k - 2's
     double S[2][M][C];
 #pragma unroll
@@ -201,7 +213,7 @@ __device__ __forceinline__ void cm_moments_segment(const CmGeom& g, int sx, int 
 #pragma unroll
         for (int l = 0; l < M; ++l) {
             double nw[C];
-            cm_apply(g, A[l], B[l], cur, nw);  // w_{l+1} of sweep row k - l - 1
+            cm_apply<C>(g, A[l], B[l], cur, nw);  // w_{l+1} of sweep row k - l - 1
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const double v = counted(nw[c], l + 1, c);
@@ -231,16 +243,16 @@ __device__ __forceinline__ void cm_moments_segment(const CmGeom& g, int sx, int 
 
 // out = q(D) b over rows [r0, r1) of strip sx, q of degree DEG with coefficients q[0 .. DEG] (shared
 // memory): a row's partial sum goes down the levels with it.
-template <int DEG>
+template <int DEG, int C>
 __device__ __forceinline__ void cm_poly_segment(const CmGeom& g, int sx, int r0, int r1, double* smem,
                                                 const double* q, double* __restrict__ out) {
-    constexpr int C = CM_C, LH = cm_halo_lanes(DEG);
+    constexpr int LH = cm_halo_lanes(DEG, C);
     const int lane = threadIdx.x & 31;
-    const int c0 = sx * cm_out(DEG) - LH * C;
+    const int c0 = sx * cm_out(DEG, C) - LH * C;
     const int h = r1 - r0;
     const int rows = h + 2 * DEG;
-    double* const stage = smem + CM_RING * CM_SLOT;
-    CmRows in(g, smem, c0, r0 - DEG, rows);
+    double* const stage = smem + CM_RING * cm_slot(C);
+    CmRows<C> in(g, smem, c0, r0 - DEG, rows);
     double S[2][DEG][C], X[DEG][C];  // X[l]: the sum up to level l of sweep row k - 1 - l
 #pragma unroll
     for (int l = 0; l < DEG; ++l)
@@ -254,7 +266,7 @@ __device__ __forceinline__ void cm_poly_segment(const CmGeom& g, int sx, int r0,
 #pragma unroll
         for (int l = 0; l < DEG; ++l) {
             double nw[C];
-            cm_apply(g, A[l], B[l], cur, nw);
+            cm_apply<C>(g, A[l], B[l], cur, nw);
             const double ql = q[l + 1];
 #pragma unroll
             for (int c = 0; c < C; ++c) {
@@ -275,7 +287,7 @@ __device__ __forceinline__ void cm_poly_segment(const CmGeom& g, int sx, int r0,
 #pragma unroll
             for (int e = 0; e < C; ++e) {
                 const int m = lane + 32 * e, i = c0 + m;
-                if (m >= LH * C && m < CM_COLS - LH * C && i < g.nx) po[i] = stage[m];
+                if (m >= LH * C && m < 32 * C - LH * C && i < g.nx) po[i] = stage[m];
             }
         }
     };
@@ -463,45 +475,56 @@ __device__ __forceinline__ void cm_publish(double (&acc)[NV], double* partials, 
 
 // The passes and sweeps are functions of their own, not inlined: each gets its registers without the
 // others' values alive around it.
-template <int M>
+template <int M, int C>
 static __device__ __noinline__ void cm_pass1(CmGeom g, int wfirst, int warps, double* smem, double* partials,
-                                         double (*red)[CM_NMU]) {
-    const CmSpan sp = cm_span(g.nx, g.ny, cm_out(M), warps, 4);
+                                             double (*red)[CM_NMU]) {
+    constexpr int LH = cm_halo_lanes(M, C), OUT = cm_out(M, C);
+    const CmSpan sp = cm_span(g.nx, g.ny, OUT, warps);
     double acc[2 * M + 1];
 #pragma unroll
     for (int v = 0; v < 2 * M + 1; ++v) acc[v] = 0.0;
     for (int w = wfirst; w < sp.n; w += warps) {
         const int sx = w % sp.strips, r0 = (w / sp.strips) * sp.seg_h, r1 = min(r0 + sp.seg_h, g.ny);
-        if ((sx + 1) * cm_out(M) <= g.nx) cm_moments_segment<M, true>(g, sx, r0, r1, smem, acc);
-        else cm_moments_segment<M, false>(g, sx, r0, r1, smem, acc);
+        if ((sx + 1) * OUT <= g.nx) cm_moments_segment<M, C, true>(g, sx, r0, r1, smem, acc);
+        else cm_moments_segment<M, C, false>(g, sx, r0, r1, smem, acc);
     }
     const int lane = threadIdx.x & 31;
-    if (lane < cm_halo_lanes(M) || lane >= 32 - cm_halo_lanes(M)) {
+    if (lane < LH || lane >= 32 - LH) {
 #pragma unroll
         for (int v = 0; v < 2 * M + 1; ++v) acc[v] = 0.0;
     }
     cm_publish<2 * M + 1>(acc, partials, red);
 }
+template <int M>
+__device__ __forceinline__ void cm_pass1_any(const CmGeom& g, int wfirst, int warps, double* smem, double* partials,
+                                             double (*red)[CM_NMU]) {
+    if (cm_narrow(g.nx, g.ny, M, warps)) cm_pass1<M, 1>(g, wfirst, warps, smem, partials, red);
+    else cm_pass1<M, CM_C>(g, wfirst, warps, smem, partials, red);
+}
 
-template <int DEG>
+template <int DEG, int C>
 static __device__ __noinline__ void cm_pass2(CmGeom g, int wfirst, int warps, double* smem, const double* q,
-                                         double* out) {
-    const CmSpan sp = cm_span(g.nx, g.ny, cm_out(DEG), warps, 4);
+                                             double* out) {
+    const CmSpan sp = cm_span(g.nx, g.ny, cm_out(DEG, C), warps);
     for (int w = wfirst; w < sp.n; w += warps) {
         const int r0 = (w / sp.strips) * sp.seg_h;
-        cm_poly_segment<DEG>(g, w % sp.strips, r0, min(r0 + sp.seg_h, g.ny), smem, q, out);
+        cm_poly_segment<DEG, C>(g, w % sp.strips, r0, min(r0 + sp.seg_h, g.ny), smem, q, out);
     }
 }
 
 // out = q(D) b over the whole grid, for a polynomial of degree deg <= CM_MAXM - 1.
 __device__ __forceinline__ void cm_pass2_any(const CmGeom& g, int deg, int wfirst, int warps, double* smem,
                                              const double* q, double* out) {
-    if (deg <= 3) cm_pass2<3>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 4) cm_pass2<4>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 5) cm_pass2<5>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 6) cm_pass2<6>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 7) cm_pass2<7>(g, wfirst, warps, smem, q, out);
-    else cm_pass2<CM_MAXM - 1>(g, wfirst, warps, smem, q, out);
+    if (cm_narrow(g.nx, g.ny, deg, warps)) {
+        if (deg <= 4) cm_pass2<4, 1>(g, wfirst, warps, smem, q, out);
+        else if (deg <= 6) cm_pass2<6, 1>(g, wfirst, warps, smem, q, out);
+        else cm_pass2<CM_MAXM - 1, 1>(g, wfirst, warps, smem, q, out);
+    } else if (deg <= 3) cm_pass2<3, CM_C>(g, wfirst, warps, smem, q, out);
+    else if (deg <= 4) cm_pass2<4, CM_C>(g, wfirst, warps, smem, q, out);
+    else if (deg <= 5) cm_pass2<5, CM_C>(g, wfirst, warps, smem, q, out);
+    else if (deg <= 6) cm_pass2<6, CM_C>(g, wfirst, warps, smem, q, out);
+    else if (deg <= 7) cm_pass2<7, CM_C>(g, wfirst, warps, smem, q, out);
+    else cm_pass2<CM_MAXM - 1, CM_C>(g, wfirst, warps, smem, q, out);
 }
 
 static __global__ void __launch_bounds__(CM_NT, 1)
@@ -551,9 +574,9 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     int mode = kCmScratch;
     if (in_range) {
         const int M = cm_levels(t);
-        if (M == 5) cm_pass1<5>(g, wfirst, warps, smem, a.partials, red);
-        else if (M == 7) cm_pass1<7>(g, wfirst, warps, smem, a.partials, red);
-        else cm_pass1<CM_MAXM>(g, wfirst, warps, smem, a.partials, red);
+        if (M == 5) cm_pass1_any<5>(g, wfirst, warps, smem, a.partials, red);
+        else if (M == 7) cm_pass1_any<7>(g, wfirst, warps, smem, a.partials, red);
+        else cm_pass1_any<CM_MAXM>(g, wfirst, warps, smem, a.partials, red);
         if (barrier()) {
             // every block adds the blocks' partials in the same order
             if (tid < 32) mu[tid] = 0.0;

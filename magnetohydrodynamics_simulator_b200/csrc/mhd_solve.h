@@ -3,6 +3,7 @@
 
 #include <algorithm>
 
+#include "mhd_cg_cluster.cuh"
 #include "mhd_cg_moments.cuh"
 #include "mhd_host_util.h"
 
@@ -12,7 +13,7 @@ struct SolveGeom {
     int strips_x = 0, seg_h = 0, nwarps = 0;  // k_cg_sweep: column strips, rows per warp, warps
     int grid = 0;                             // k_cg_sweep's blocks
     int mgrid = 0;                            // k_solve's blocks
-    bool small = false;                       // k_solve alone, whatever the matrix
+    int cluster = 0;                          // k_cg_cluster's blocks; 0: the grid does not fit a cluster
     // doubles of the partial sums of either kernel
     size_t partials() const {
         return std::max((size_t)2 * grid * 4, (size_t)mgrid * (mhd::CM_NMU + 8));
@@ -34,6 +35,8 @@ inline mhd_status solve_setup() {
         MHD_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, mhd::CGS_NT, mhd::kCgRingBytes));
         if (occ < 1) return MHD_ERR_CUDA;
     }
+    MHD_TRY(cudaFuncSetAttribute(mhd::k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(mhd::CC_SMEM_DOUBLES * sizeof(double))));
     MHD_TRY(cudaFuncSetAttribute(mhd::k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)mhd::kCmSmemBytes));
     MHD_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mhd::k_solve, mhd::CM_NT, mhd::kCmSmemBytes));
@@ -50,11 +53,14 @@ inline SolveGeom solve_geometry(int nx, int ny, int num_sms) {
     const int segs = std::max(1, g.grid * NW / g.strips_x);
     g.seg_h = std::max(4, (ny + segs - 1) / segs);
     g.nwarps = g.strips_x * ((ny + g.seg_h - 1) / g.seg_h);
-    // k_solve: segments of 4 rows or more, two per block until every SM has a block
-    const int out = mhd::cm_out(mhd::CM_MAXM);
+    // k_solve: narrow segments of 4 rows or more, four per block until every SM has a block
+    const int out = mhd::cm_out(mhd::CM_MAXM, 1);
     const long long nseg = (long long)((nx + out - 1) / out) * ((ny + 3) / 4);
-    g.mgrid = (int)std::max(1LL, std::min((long long)num_sms, (nseg + 1) / 2));
-    g.small = (long long)nx * ny <= 256 * 256;
+    g.mgrid = (int)std::max(1LL, std::min((long long)num_sms, (nseg + 3) / 4));
+    // the largest cluster whose bands have at least one row
+    int cs = mhd::CC_MAX;
+    while (cs > 1 && ny < cs) cs /= 2;
+    g.cluster = mhd::cc_fits(nx, ny, cs) ? cs : 0;
     return g;
 }
 
@@ -68,11 +74,28 @@ inline double solve_t(double alpha, double dx, double dy) {
 // over the face planes), beyond it k_cg_sweep alone (one sweep per product). Where the host does not
 // know, k_solve comes first and k_cg_sweep behind it finds the solve done, or does it: an idle kernel
 // costs 1 us, the sweeps on k_solve's half as many warps a quarter more time (1024^2: 188 against 150 us).
-// Small grids, whose t is small (it grows with eta / dx under the CFL rule), take k_solve alone.
-inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, SolveSync* dev, cudaStream_t stream) {
+// Grids that fit one cluster take k_cg_cluster, whatever the matrix.
+// field: the right-hand side is a caller's field, not an evolved one. Smooth fields take two to four products,
+// and below 1448^2 as many sweeps are shorter than the two passes, whose length does not depend on them
+// (1024^2: 3 products 66 against 76 us; 2048^2: 198 against 154); in a step there are five or more.
+inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool field, SolveSync* dev,
+                               cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
+    if (g.cluster) {
+        cfg.gridDim = dim3(g.cluster);
+        cfg.blockDim = dim3(mhd::CC_NT);
+        cfg.dynamicSmemBytes =
+            (size_t)mhd::cc_smem_doubles(a.D.nx, (a.D.ny + g.cluster - 1) / g.cluster) * sizeof(double);
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = g.cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        MHD_TRY(cudaLaunchKernelEx(&cfg, mhd::k_cg_cluster, a));
+        return MHD_OK;
+    }
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
@@ -80,9 +103,10 @@ inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t,
     a.strips_x = g.strips_x;
     a.seg_h = g.seg_h;
     a.nwarps = g.nwarps;
-    const bool sweep = t > mhd::kCmMaxT || (t < 0.0 && !g.small);
+    const bool moments = t <= mhd::kCmMaxT && !(field && (long long)a.D.nx * a.D.ny < (1 << 21));
+    const bool sweep = t < 0.0 || !moments;
     a.start = (t < 0.0 && sweep) ? &dev->start : nullptr;
-    if (t <= mhd::kCmMaxT) {
+    if (moments) {
         a.sync = &dev->sync[0];
         cfg.gridDim = dim3(g.mgrid);
         cfg.blockDim = dim3(mhd::CM_NT);

@@ -1,6 +1,6 @@
-"""The implicit solve's forms -- two passes from moments, the ordinary CG sweeps, and the hand-over from
-one to the other -- at the sizes where their strips and segments end, through mhd_resistive_rate and
-mhd_step.
+"""The implicit solve's forms -- one cluster with everything in shared memory, two passes from moments,
+the ordinary CG sweeps, and the hand-over from one to the other -- at the sizes where their strips, bands
+and segments end, through mhd_resistive_rate and mhd_step.
 
 Reference: plain numpy CG (x0 = 0, constant Jacobi diagonal, stop when |r|^2 < eps^2 |b|^2: the
 reference's solver, solvers.hpp:404-489 with Eigen's defaults) on the same right-hand side. Both
@@ -76,9 +76,10 @@ def _rate(m, nx, ny, dx, dy, eta, alpha, bx, by, **kw):
     return ox.cpu().numpy(), oy.cpu().numpy(), prods, status
 
 
-# grids below, at and above a strip's output columns (84 and 78) and a segment's 4 rows, odd and tiny ones;
-# t = 2 alpha (1/dx^2 + 1/dy^2) in each variant's range, below the limit of the moment form and above it
-@pytest.mark.parametrize("shape", [(2, 2), (3, 5), (78, 4), (79, 9), (84, 33), (85, 64), (157, 131), (300, 290)])
+# clusters of 1 .. 8 blocks with bands of one row and more, one cell or runs of four rows a thread, odd
+# widths, the largest that fits (181 x 181) and the first that does not; a grid for the sweeps
+@pytest.mark.parametrize("shape", [(2, 2), (3, 5), (78, 4), (79, 9), (84, 33), (85, 64), (1021, 8), (157, 131), (181, 181),
+                                   (182, 181), (300, 290)])
 @pytest.mark.parametrize("t,kind", [(4e-4, "smooth"), (4e-4, "noise"), (8e-3, "rough"), (1.4e-2, "noise"), (4e-2, "rough"),
                                     (5.5e-2, "noise"), (0.3, "rough"), (2.0, "noise")])
 def test_rate_matches_plain_cg(m, shape, t, kind):
@@ -119,6 +120,52 @@ def test_loose_tolerance_stops_early(m):
     assert few[3] == full[3] == 0 and 0 < few[2] < full[2]
     # |r| < 1e-6 |b| and the matrix's smallest eigenvalue is 1
     assert np.linalg.norm(few[0] - full[0]) <= 1e-5 * np.linalg.norm(full[0])
+
+
+# the moment form through a step of fixed dt (U* = U where nothing moves: rho = p = 1, v = 0 and a field so
+# weak that the explicit stage leaves its faces alone to rounding): widths below, at and above a strip's
+# output columns (84, 78 with three columns a lane; 22, 18, 14 with one), t in each variant's range
+@pytest.mark.parametrize("shape", [(234, 200), (235, 211), (252, 180), (253, 190), (700, 61), (1030, 47), (1500, 260)])
+@pytest.mark.parametrize("t,kind", [(4e-4, "smooth"), (8e-3, "rough"), (1.4e-2, "noise"), (4e-2, "rough"), (5.5e-2, "noise")])
+def test_step_in_moment_form_matches_plain_cg(m, shape, t, kind):
+    nx, ny = shape
+    dx, dy = 2 * np.pi / nx, 1.3 * 2 * np.pi / ny
+    dt = 1e-9
+    g = m.ars_gamma()
+    eta = t / (2 * (1 / dx**2 + 1 / dy**2)) / (dt * g)
+    bx, by = _faces(nx, ny, dx, dy, kind, seed=nx * 31 + ny)
+    scale = 1e-6 / max(np.abs(bx).max(), np.abs(by).max())
+    bx, by = scale * bx, scale * by
+    one, zero = np.ones((ny, nx)), np.zeros((ny, nx))
+    ctx = m.Context(nx, ny, dx, dy, eta)
+    ctx.set_state([one, zero, zero, 1.5 * one, bx, by])
+    ctx.step(dt)
+    assert ctx.synchronize_status() == 0
+    got, prods = ctx.get_state(), ctx.last_cg_products()
+    ctx.close()
+    # the step's linear part (solvers.hpp:491-613 without the explicit rates)
+    alpha = dt * eta * g
+
+    def curl(e):
+        return -(np.roll(e, -1, 0) - e) / dy, (np.roll(e, -1, 1) - e) / dx
+
+    def jz(u, v):
+        return eta * ((v - np.roll(v, 1, 1)) / dx - (u - np.roll(u, 1, 0)) / dy)
+
+    x1, k1 = _cg(bx, by, dx, dy, eta, alpha)
+    r = curl(x1)
+    b1 = bx + dt * g * r[0], by + dt * g * r[1]
+    r = curl(jz(*b1))
+    a = bx + dt * (1 - g) * r[0], by + dt * (1 - g) * r[1]
+    x2, k2 = _cg(*a, dx, dy, eta, alpha)
+    r = curl(x2)
+    r = curl(jz(a[0] + dt * g * r[0], a[1] + dt * g * r[1]))
+    want = a[0] + dt * g * r[0], a[1] + dt * g * r[1]
+    assert abs(prods[0] - k1) <= 1 and abs(prods[1] - k2) <= 1, (prods, k1, k2)
+    # the implicit increments dt g curl(x) are t |B| or less, known to 64 eps as in the rates above; sums and
+    # the explicit stage (numerical diffusion dt c / h < 1e-6 of B's variation from cell to cell) on top
+    bound = (64 * EPS + 2e-6 * dt * 2 * np.sqrt(5 / 3) / min(dx, dy) / 1e-6) * 1e-6 * 4
+    assert max(np.abs(got[4] - want[0]).max(), np.abs(got[5] - want[1]).max()) <= bound
 
 
 @pytest.mark.parametrize("t,noise", [(0.15, 0.0), (0.05, 0.3)])
