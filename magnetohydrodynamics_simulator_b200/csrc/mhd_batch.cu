@@ -17,7 +17,7 @@
 #include <new>
 #include <vector>
 
-#include "mhd_batch.cuh"
+#include "mhd_batch_solve.cuh"
 #include "mhd_host_util.h"
 
 using namespace mhd;
@@ -65,7 +65,21 @@ struct mhd_batch {
     int stage_occ[2] = {0, 0}, fin_occ = 0, cg_occ = 0;
     int stage_grid[2] = {0, 0}, fin_grid = 0, cg_grid = 0;
     double* partials = nullptr;  // [2][CGB_MAX_INST][cg_occ * num_sms][4]
-    CgSync* syncs = nullptr;     // [2 * nchunks]
+    CgSync* syncs = nullptr;     // [2 * nchunks] of k_cg_batch
+    // solves (mhd_batch_solve.cuh), by chunk: instances that take a cluster, and all others
+    struct SolveLists {
+        std::vector<int> cluster, big;
+        int cluster_off = 0, big_off = 0;  // in d_lists
+    };
+    std::vector<SolveLists> lists;
+    int cluster_blocks = 0;
+    size_t cluster_smem = 0;
+    int solve_grid = 0;
+    int* d_lists = nullptr;
+    int* todo = nullptr;             // [count]
+    BatchPlan* plans = nullptr;      // [CGB_MAX_INST]
+    double* tile_partials = nullptr;
+    CgSync* solve_syncs = nullptr;   // [nchunks] of k_solve_batch
     int* queues = nullptr;       // [kQueues]
     double* dt_dev = nullptr;    // [count] per-instance dt of mhd_batch_step
     double* divb_partial = nullptr;
@@ -210,8 +224,101 @@ mhd_status apply_tuning(mhd_batch* b, const mhd_batch_tuning& t) {
     return MHD_OK;
 }
 
+// Which instances' solves run in a cluster: those of at most CC's cells, in clusters of the fewest blocks that
+// hold the largest of them, or of more while all clusters are resident at once. More than two waves of clusters
+// take longer than the moment form: then the largest instances go there.
+void plan_solves(mhd_batch* b) {
+    std::vector<int> small;
+    auto fits = [&](int i, int cs) { return cc_fits(b->prm[i].nx, b->prm[i].ny, cs); };
+    for (int i = 0; i < b->count; ++i)
+        if (fits(i, std::min(CC_MAX, b->prm[i].ny >= 8 ? 8 : (b->prm[i].ny >= 4 ? 4 : 1)))) small.push_back(i);
+    std::stable_sort(small.begin(), small.end(), [&](int x, int y) { return b->ncell[x] > b->ncell[y]; });
+    int cs = 0;
+    while (!small.empty()) {
+        cs = 1;
+        auto all_fit = [&](int c) {
+            for (int i : small)
+                if (!fits(i, c)) return false;
+            return true;
+        };
+        while (cs < CC_MAX && !all_fit(cs)) cs *= 2;
+        if (all_fit(cs) && (long long)small.size() * cs <= 2LL * b->num_sms) break;
+        small.erase(small.begin());
+    }
+    if (!small.empty()) {
+        auto all_fit = [&](int c) {
+            for (int i : small)
+                if (!fits(i, c)) return false;
+            return true;
+        };
+        while (cs < CC_MAX && (long long)small.size() * cs * 2 <= b->num_sms && all_fit(2 * cs)) cs *= 2;
+    }
+    b->cluster_blocks = cs;
+    b->cluster_smem = 0;
+    std::vector<char> in_cluster(b->count, 0);
+    for (int i : small) {
+        in_cluster[i] = 1;
+        const int R = (b->prm[i].ny + cs - 1) / cs;
+        b->cluster_smem = std::max(b->cluster_smem, (size_t)cc_smem_doubles(b->prm[i].nx, R) * sizeof(double));
+    }
+    b->lists.assign(b->nchunks, mhd_batch::SolveLists{});
+    int off = 0;
+    for (int c = 0; c < b->nchunks; ++c) {
+        mhd_batch::SolveLists& L = b->lists[c];
+        for (int i = c * CGB_MAX_INST; i < std::min(b->count, (c + 1) * CGB_MAX_INST); ++i)
+            (in_cluster[i] ? L.cluster : L.big).push_back(i);
+        L.cluster_off = off;
+        off += (int)L.cluster.size();
+        L.big_off = off;
+        off += (int)L.big.size();
+    }
+}
+
 mhd_status launch_cg_chunks(mhd_batch* b, const BatchInst* insts, int solve, bool record) {
     for (int c = 0; c < b->nchunks; ++c) {
+        const mhd_batch::SolveLists& L = b->lists[c];
+        if (!L.cluster.empty()) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)L.cluster.size() * b->cluster_blocks);
+            cfg.blockDim = dim3(CC_NT);
+            cfg.dynamicSmemBytes = b->cluster_smem;
+            cfg.stream = b->stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = b->cluster_blocks;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            MHD_TRY(cudaLaunchKernelEx(&cfg, k_cluster_batch, insts, (const int*)(b->d_lists + L.cluster_off),
+                                       b->cluster_blocks, solve, b->rec_cap, record ? b->rec_prods : nullptr,
+                                       b->timeout_s));
+        }
+        if (L.big.empty()) continue;
+        {
+            SolveBatchArgs a{};
+            a.insts = insts;
+            a.list = b->d_lists + L.big_off;
+            a.n = (int)L.big.size();
+            a.solve = solve;
+            a.partials = b->tile_partials;
+            a.plans = b->plans;
+            a.todo = b->todo;
+            a.sync = b->solve_syncs + c;
+            a.rec_stride = b->rec_cap;
+            a.prods_rec = record ? b->rec_prods : nullptr;
+            a.timeout_s = b->timeout_s;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(b->solve_grid);
+            cfg.blockDim = dim3(CM_NT);
+            cfg.dynamicSmemBytes = kCmSmemBytes;
+            cfg.stream = b->stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            MHD_TRY(cudaLaunchKernelEx(&cfg, k_solve_batch, a));
+        }
         CgBatchArgs a{};
         a.insts = insts;
         a.inst0 = c * CGB_MAX_INST;
@@ -220,6 +327,7 @@ mhd_status launch_cg_chunks(mhd_batch* b, const BatchInst* insts, int solve, boo
         a.rows = b->tuning.cg_rows;
         a.partials = b->partials;
         a.sync = b->syncs + 2 * c + solve;
+        a.todo = b->todo;
         a.solve_index = solve;
         a.rec_stride = b->rec_cap;
         a.prods_rec = record ? b->rec_prods : nullptr;
@@ -370,6 +478,26 @@ mhd_status mhd_batch_create(const mhd_params* params, int count, void* stream, m
         cudaGetLastError();
         return fail(MHD_ERR_CUDA);
     }
+    plan_solves(b);
+    int solve_occ = 0;
+    if (cudaFuncSetAttribute(k_solve_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCmSmemBytes) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_cluster_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(CC_SMEM_DOUBLES * sizeof(double))) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&solve_occ, k_solve_batch, CM_NT, kCmSmemBytes) != cudaSuccess ||
+        solve_occ < 1) {
+        cudaGetLastError();
+        return fail(MHD_ERR_CUDA);
+    }
+    long long max_tiles = 1;  // of any chunk's passes, at the lowest tiles
+    for (const mhd_batch::SolveLists& L : b->lists) {
+        long long n = 0;
+        for (int i : L.big)
+            n += (long long)((b->prm[i].nx + cm_out(CM_MAXM, CM_C) - 1) / cm_out(CM_MAXM, CM_C)) *
+                 ((b->prm[i].ny + kCmTileMinRows - 1) / kCmTileMinRows);
+        max_tiles = std::max(max_tiles, n);
+    }
+    b->solve_grid = (int)std::min((long long)b->num_sms, (max_tiles + 3) / 4);
     b->cg_occ = std::min(b->cg_occ, std::max(1, mhd_host::env_int("MHD_B200_CG_BLOCKS_PER_SM", 1)));
     const size_t max_cg_grid = (size_t)b->cg_occ * b->num_sms;
     size_t max_cells = 0;
@@ -383,6 +511,11 @@ mhd_status mhd_batch_create(const mhd_params* params, int count, void* stream, m
         cudaMalloc(&b->partials, 2 * (size_t)CGB_MAX_INST * max_cg_grid * 4 * sizeof(double)) !=
             cudaSuccess ||
         cudaMalloc(&b->syncs, 2 * (size_t)b->nchunks * sizeof(CgSync)) != cudaSuccess ||
+        cudaMalloc(&b->d_lists, count * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&b->todo, count * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&b->plans, CGB_MAX_INST * sizeof(BatchPlan)) != cudaSuccess ||
+        cudaMalloc(&b->tile_partials, (size_t)max_tiles * CM_NMU * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&b->solve_syncs, (size_t)b->nchunks * sizeof(CgSync)) != cudaSuccess ||
         cudaMalloc(&b->queues, kQueues * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&b->dt_dev, count * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&b->divb_partial, 2 * (size_t)b->divb_blocks * sizeof(double)) != cudaSuccess ||
@@ -457,8 +590,17 @@ mhd_status mhd_batch_create(const mhd_params* params, int count, void* stream, m
         cudaMemsetAsync(b->pool, 0, (size_t)kBatchPlanes * b->total_cells * sizeof(double),
                         b->stream) != cudaSuccess ||
         cudaMemsetAsync(b->syncs, 0, 2 * (size_t)b->nchunks * sizeof(CgSync), b->stream) !=
-            cudaSuccess)
+            cudaSuccess ||
+        cudaMemsetAsync(b->solve_syncs, 0, (size_t)b->nchunks * sizeof(CgSync), b->stream) != cudaSuccess ||
+        cudaMemsetAsync(b->todo, 0, count * sizeof(int), b->stream) != cudaSuccess)
         return fail(MHD_ERR_CUDA);
+    for (const mhd_batch::SolveLists& L : b->lists) {
+        if (cudaMemcpy(b->d_lists + L.cluster_off, L.cluster.data(), L.cluster.size() * sizeof(int),
+                       cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(b->d_lists + L.big_off, L.big.data(), L.big.size() * sizeof(int), cudaMemcpyHostToDevice) !=
+                cudaSuccess)
+            return fail(MHD_ERR_CUDA);
+    }
     mhd_batch_tuning t{};
     t.stage_rows = mhd_host::env_int("MHD_B200_BATCH_STAGE_ROWS", balanced_stage_rows(b, 2));
     t.stage_tail_rows = mhd_host::env_int("MHD_B200_BATCH_STAGE_TAIL_ROWS", 0);
@@ -482,6 +624,11 @@ mhd_status mhd_batch_destroy(mhd_batch* b) {
     cudaFree(b->d_items_mem);
     cudaFree(b->partials);
     cudaFree(b->syncs);
+    cudaFree(b->d_lists);
+    cudaFree(b->todo);
+    cudaFree(b->plans);
+    cudaFree(b->tile_partials);
+    cudaFree(b->solve_syncs);
     cudaFree(b->queues);
     cudaFree(b->dt_dev);
     cudaFree(b->divb_partial);
@@ -500,7 +647,12 @@ int mhd_batch_count(mhd_batch* b) { return b ? b->count : 0; }
 
 void* mhd_batch_stream(mhd_batch* b) { return b ? (void*)b->stream : nullptr; }
 
-int mhd_batch_launches_per_step(mhd_batch* b) { return b ? 4 + 2 * b->nchunks : 0; }
+int mhd_batch_launches_per_step(mhd_batch* b) {
+    if (!b) return 0;
+    int n = 4;  // coefficients, two stages, finalize; twice the chunks' solves
+    for (const mhd_batch::SolveLists& L : b->lists) n += 2 * ((L.cluster.empty() ? 0 : 1) + (L.big.empty() ? 0 : 2));
+    return n;
+}
 
 static mhd_status batch_copy_in(mhd_batch* b, int index, const double* const f[6],
                                 cudaMemcpyKind kind) {
@@ -769,6 +921,8 @@ mhd_status mhd_batch_synchronize(mhd_batch* b, mhd_status* per_instance) {
         any |= b->host_status[i].flags != 0;
     }
     if (any) {
+        if (worst == MHD_ERR_TIMEOUT)
+            MHD_TRY(cudaMemsetAsync(b->solve_syncs, 0, (size_t)b->nchunks * sizeof(CgSync), b->stream));
         for (int i = 0; i < b->count; ++i)
             if (b->host_status[i].flags)
                 MHD_TRY(cudaMemsetAsync(&b->status[i].flags, 0, sizeof(unsigned int), b->stream));

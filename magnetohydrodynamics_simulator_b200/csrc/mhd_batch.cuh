@@ -179,8 +179,8 @@ k_finalize_batch(const BatchInst* __restrict__ insts, const SweepItem* __restric
 }
 
 // ------------------------------------------------------------------------------------------
-// Batched implicit solve: the CGs of up to CGB_MAX_INST instances in one persistent cooperative
-// kernel, running their phases in lockstep (solvers.hpp:404-489 per instance, Eigen's
+// Batched implicit solve, the ordinary iterations (for what the forms of mhd_batch_solve.cuh leave): the CGs
+// of up to CGB_MAX_INST instances in one persistent cooperative kernel, running their phases in lockstep (solvers.hpp:404-489 per instance, Eigen's
 // ConjugateGradient defaults as in k_cg_sweep).
 //
 // In every phase the work of the instances still iterating is numbered 0 .. T-1 through a prefix
@@ -211,7 +211,8 @@ constexpr int CGB_NW = CGB_NT / 32;
 constexpr size_t kCgbRingBytes = (size_t)CGB_NW * CG_RING * CG_SLOT * sizeof(double);
 constexpr size_t kCgbSmemBytes = kCgbRingBytes + (size_t)CGB_NW * CGB_MAX_INST * 4 * sizeof(double);
 
-enum CgInstStatus : int { kCgActive = 0, kCgConverged = 1, kCgZero = 2, kCgBreakdown = 3, kCgCapped = 4 };
+enum CgInstStatus : int { kCgActive = 0, kCgConverged = 1, kCgZero = 2, kCgBreakdown = 3, kCgCapped = 4,
+                          kCgSolved = 5 };  // before this kernel
 
 struct CgBInst {
     double cx, cy, diag, invdiag;  // matrix of this solve
@@ -230,6 +231,7 @@ struct CgBatchArgs {
     int rows;                // order 1 with rows = 0: the tile height is chosen phase by phase
     double* partials;        // [2][CGB_MAX_INST][gridDim.x][4]
     CgSync* sync;
+    const int* todo;         // [count]: instances that k_solve_batch left to this kernel
     int solve_index;         // 0: B* = U1*_B (T planes), 1: B* = U2*_B (A planes)
     int rec_stride;
     long long* prods_rec;    // [instance][rec_stride][2] products record, or null
@@ -448,6 +450,9 @@ k_cg_batch(CgBatchArgs a) {
         return false;
     };
 
+    int left = 0;
+    for (int li = tid; li < a.ninst; li += CGB_NT) left |= a.todo[a.inst0 + li];
+    if (!__syncthreads_or(left)) return;
     // matrix of each instance's solve (the coefficient was set by this step's coefficients)
     for (int li = tid; li < a.ninst; li += CGB_NT) {
         const BatchInst& I = a.insts[a.inst0 + li];
@@ -462,7 +467,7 @@ k_cg_batch(CgBatchArgs a) {
         S.beta = 0.0;
         S.products = 0;
         S.rr = 0.0;
-        S.status = kCgActive;
+        S.status = a.todo[a.inst0 + li] ? kCgActive : kCgSolved;
         S.ny = I.D.ny;
         S.strips = I.cg_strips_x;
     }
@@ -474,6 +479,7 @@ k_cg_batch(CgBatchArgs a) {
     cgb_phase<0, 3>(a, sh, pref, h, wsum, ring, 0, dir, part(phase));
     if (!barrier_or_quit()) return;
     for (int li = wid; li < a.ninst; li += NW) {
+        if (sh[li].status != kCgActive) continue;
         double v[3];
         cgb_span_sum<3>(part(phase), li, v);
         if (lane == 0) {
@@ -568,6 +574,7 @@ k_cg_batch(CgBatchArgs a) {
         for (int li = tid; li < a.ninst; li += CGB_NT) {
             const BatchInst& I = a.insts[a.inst0 + li];
             const CgBInst& S = sh[li];
+            if (S.status == kCgSolved) continue;
             I.st->cg_products[a.solve_index] = S.products;
             I.st->cg_products_sum[a.solve_index] += S.products;
             I.st->cg_last_rr[a.solve_index] = (S.bb > 0.0) ? S.rr / S.bb : 0.0;

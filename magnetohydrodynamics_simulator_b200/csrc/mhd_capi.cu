@@ -463,8 +463,9 @@ mhd_status mhd_destroy(mhd_context* c) {
 void* mhd_stream(mhd_context* c) { return c ? (void*)c->stream : nullptr; }
 
 int mhd_launches_per_step(mhd_context* c) {
-    (void)c;
-    return 6;  // coefficients, stage 1, CG, stage 2, CG, finalize
+    // coefficients, stage 1, solve, stage 2, solve, finalize; a CFL step's solves on a grid that does not fit a
+    // cluster are two kernels each (mhd_host::launch_solve)
+    return (c && c->solve.cluster == 0) ? 8 : 6;
 }
 
 // Work about to write the state planes waits for the copies of mhd_get_state_async.

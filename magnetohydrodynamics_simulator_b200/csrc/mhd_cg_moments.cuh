@@ -93,6 +93,17 @@ struct CmGeom {
     const double* byf;
 };
 
+// This warp's shared memory. The functions that are not inlined ask for it themselves: a pointer argument
+// would be a generic address, and every access through it one of the slower generic loads and stores.
+__device__ __forceinline__ double* cm_warp_smem() {
+#if defined(__CUDA_ARCH__)
+    extern __shared__ __align__(16) double cm_mem[];
+#else
+    static double cm_mem[kCmSmemBytes / sizeof(double)];
+#endif
+    return cm_mem + (size_t)(threadIdx.x >> 5) * CM_WARP;
+}
+
 // A warp's stream of right-hand-side rows: cp.async into the ring, coalesced; each lane then reads
 // its C adjacent columns. Sweep row k holds grid row j0 + k (k = -1: only bx, the row below the
 // first). The caller runs next() once per row, in order.
@@ -476,9 +487,10 @@ __device__ __forceinline__ void cm_publish(double (&acc)[NV], double* partials, 
 // The passes and sweeps are functions of their own, not inlined: each gets its registers without the
 // others' values alive around it.
 template <int M, int C>
-static __device__ __noinline__ void cm_pass1(CmGeom g, int wfirst, int warps, double* smem, double* partials,
+static __device__ __noinline__ void cm_pass1(CmGeom g, int wfirst, int warps, double* partials,
                                              double (*red)[CM_NMU]) {
     constexpr int LH = cm_halo_lanes(M, C), OUT = cm_out(M, C);
+    double* const smem = cm_warp_smem();
     const CmSpan sp = cm_span(g.nx, g.ny, OUT, warps);
     double acc[2 * M + 1];
 #pragma unroll
@@ -496,15 +508,16 @@ static __device__ __noinline__ void cm_pass1(CmGeom g, int wfirst, int warps, do
     cm_publish<2 * M + 1>(acc, partials, red);
 }
 template <int M>
-__device__ __forceinline__ void cm_pass1_any(const CmGeom& g, int wfirst, int warps, double* smem, double* partials,
+__device__ __forceinline__ void cm_pass1_any(const CmGeom& g, int wfirst, int warps, double* partials,
                                              double (*red)[CM_NMU]) {
-    if (cm_narrow(g.nx, g.ny, M, warps)) cm_pass1<M, 1>(g, wfirst, warps, smem, partials, red);
-    else cm_pass1<M, CM_C>(g, wfirst, warps, smem, partials, red);
+    if (cm_narrow(g.nx, g.ny, M, warps)) cm_pass1<M, 1>(g, wfirst, warps, partials, red);
+    else cm_pass1<M, CM_C>(g, wfirst, warps, partials, red);
 }
 
 template <int DEG, int C>
-static __device__ __noinline__ void cm_pass2(CmGeom g, int wfirst, int warps, double* smem, const double* q,
+static __device__ __noinline__ void cm_pass2(CmGeom g, int wfirst, int warps, const double* q,
                                              double* out) {
+    double* const smem = cm_warp_smem();
     const CmSpan sp = cm_span(g.nx, g.ny, cm_out(DEG, C), warps);
     for (int w = wfirst; w < sp.n; w += warps) {
         const int r0 = (w / sp.strips) * sp.seg_h;
@@ -513,18 +526,18 @@ static __device__ __noinline__ void cm_pass2(CmGeom g, int wfirst, int warps, do
 }
 
 // out = q(D) b over the whole grid, for a polynomial of degree deg <= CM_MAXM - 1.
-__device__ __forceinline__ void cm_pass2_any(const CmGeom& g, int deg, int wfirst, int warps, double* smem,
+__device__ __forceinline__ void cm_pass2_any(const CmGeom& g, int deg, int wfirst, int warps,
                                              const double* q, double* out) {
     if (cm_narrow(g.nx, g.ny, deg, warps)) {
-        if (deg <= 4) cm_pass2<4, 1>(g, wfirst, warps, smem, q, out);
-        else if (deg <= 6) cm_pass2<6, 1>(g, wfirst, warps, smem, q, out);
-        else cm_pass2<CM_MAXM - 1, 1>(g, wfirst, warps, smem, q, out);
-    } else if (deg <= 3) cm_pass2<3, CM_C>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 4) cm_pass2<4, CM_C>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 5) cm_pass2<5, CM_C>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 6) cm_pass2<6, CM_C>(g, wfirst, warps, smem, q, out);
-    else if (deg <= 7) cm_pass2<7, CM_C>(g, wfirst, warps, smem, q, out);
-    else cm_pass2<CM_MAXM - 1, CM_C>(g, wfirst, warps, smem, q, out);
+        if (deg <= 4) cm_pass2<4, 1>(g, wfirst, warps, q, out);
+        else if (deg <= 6) cm_pass2<6, 1>(g, wfirst, warps, q, out);
+        else cm_pass2<CM_MAXM - 1, 1>(g, wfirst, warps, q, out);
+    } else if (deg <= 3) cm_pass2<3, CM_C>(g, wfirst, warps, q, out);
+    else if (deg <= 4) cm_pass2<4, CM_C>(g, wfirst, warps, q, out);
+    else if (deg <= 5) cm_pass2<5, CM_C>(g, wfirst, warps, q, out);
+    else if (deg <= 6) cm_pass2<6, CM_C>(g, wfirst, warps, q, out);
+    else if (deg <= 7) cm_pass2<7, CM_C>(g, wfirst, warps, q, out);
+    else cm_pass2<CM_MAXM - 1, CM_C>(g, wfirst, warps, q, out);
 }
 
 static __global__ void __launch_bounds__(CM_NT, 1)
@@ -534,11 +547,6 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     __shared__ double scal[8];
     __shared__ CmPlan plan;
     __shared__ int sflag;
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double cm_mem[];
-#else
-    static double cm_mem[kCmSmemBytes / sizeof(double)];
-#endif
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     CgScal s = cg_scalars(a);
     const double t = 2 * (s.cx + s.cy);
@@ -550,7 +558,6 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     const int G = gridDim.x, warps = G * CM_NW;
     // consecutive segments go to different SMs, so that few of them spread out
     const int wfirst = wid * G + blockIdx.x;
-    double* const smem = cm_mem + (size_t)wid * CM_WARP;
     unsigned long long target = barrier_base(a.sync);
     const unsigned long long deadline = global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
     CmGeom g;
@@ -574,9 +581,9 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     int mode = kCmScratch;
     if (in_range) {
         const int M = cm_levels(t);
-        if (M == 5) cm_pass1_any<5>(g, wfirst, warps, smem, a.partials, red);
-        else if (M == 7) cm_pass1_any<7>(g, wfirst, warps, smem, a.partials, red);
-        else cm_pass1_any<CM_MAXM>(g, wfirst, warps, smem, a.partials, red);
+        if (M == 5) cm_pass1_any<5>(g, wfirst, warps, a.partials, red);
+        else if (M == 7) cm_pass1_any<7>(g, wfirst, warps, a.partials, red);
+        else cm_pass1_any<CM_MAXM>(g, wfirst, warps, a.partials, red);
         if (barrier()) {
             // every block adds the blocks' partials in the same order
             if (tid < 32) mu[tid] = 0.0;
@@ -593,7 +600,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
             __syncthreads();
             mode = plan.mode;
             if (mode == kCmDone || mode == kCmCapped || mode == kCmContinue)
-                cm_pass2_any(g, plan.k - 1, wfirst, warps, smem, plan.q, a.x);
+                cm_pass2_any(g, plan.k - 1, wfirst, warps, plan.q, a.x);
         }
     }
     CgResult res{};
@@ -602,8 +609,8 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
         CgStart start{};
         if (mode == kCmContinue) {
             // r_k into the buffer iteration k reads, p_{k-1} likewise (k is odd)
-            cm_pass2_any(g, plan.k, wfirst, warps, smem, plan.qr, a.r[1]);
-            cm_pass2_any(g, plan.k - 1, wfirst, warps, smem, plan.qp, a.p[0]);
+            cm_pass2_any(g, plan.k, wfirst, warps, plan.qr, a.r[1]);
+            cm_pass2_any(g, plan.k - 1, wfirst, warps, plan.qp, a.p[0]);
             start.k = plan.k;
             start.alpha = plan.alpha;
             start.alpha_prev = plan.alpha_prev;
@@ -624,7 +631,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
                 const int seg_h = max(4, (g.ny + segs - 1) / segs);
                 // (partials of its own: other blocks may still read the moments')
                 cg_iterate<CM_NT, false, true>(a, strips, seg_h, strips * ((g.ny + seg_h - 1) / seg_h), s,
-                                  cm_mem + (size_t)wid * CG_RING * CG_SLOT, a.partials + (size_t)CM_NMU * G, &red[0][0],
+                                  cm_warp_smem(), a.partials + (size_t)CM_NMU * G, &red[0][0],
                                   scal, barrier, start, res);
             }
             report = alive;
