@@ -44,7 +44,7 @@ using namespace mhd;
 namespace {
 
 constexpr int kSlotPlanes = 14;     // T[6], A[6], Bn[2]
-constexpr int kScratchPlanes = 59;  // adjoint-step and solver scratch (see AdjScratch)
+constexpr int kScratchPlanes = 58;  // adjoint-step and solver scratch (see AdjScratch)
 
 struct Slot {
     double* T[6];
@@ -57,8 +57,7 @@ struct AdjScratch {
     double* lamT[6];  // adjoint of the predictor
     double* w[6];     // rate adjoint handed to F'^T
     double* fb[2];    // face-B temporaries
-    double* c1;       // corner temporaries
-    double* c2;
+    double* c2;       // corner current (Jz of B2, then of B1)
     double* B1[2];    // B1 = T_B + cg C(x1)
     double* y;        // solver solution / adjoint solve
     double* r[2];
@@ -97,7 +96,6 @@ struct mhd_adjoint {
     SweepGeom sg[2]{}, fg{};
     int st_blocks[2]{}, fn_blocks = 0;
     mhd_host::SolveGeom geom;  // implicit solve
-    int ew_blocks = 0, dot_blocks = 0;
     bool have_forward = false;
 };
 
@@ -193,18 +191,15 @@ mhd_status copy_planes(mhd_adjoint* a, double* const dst[6], const double* const
     return MHD_OK;
 }
 
-// geta += scale * sum(x * y)
-mhd_status dot_acc(mhd_adjoint* a, const double* x, const double* y, double scale) {
-    k_adj_dot_partial<<<a->dot_blocks, 256, 0, a->stream>>>(a->n, x, y, a->dot_partial);
-    MHD_TRY(cudaGetLastError());
-    k_adj_dot_final<<<1, 32, 0, a->stream>>>(a->dot_partial, a->dot_blocks, scale, a->geta);
-    MHD_TRY(cudaGetLastError());
-    return MHD_OK;
+// Launch shape of the resistive kernels: columns on x, rows strided over about eight blocks an SM.
+dim3 adj_grid(const mhd_adjoint* a) {
+    const int gx = (a->dom.nx + 255) / 256;
+    return dim3((unsigned)gx, (unsigned)std::max(1, std::min(a->dom.ny, (a->num_sms * 8 + gx - 1) / gx)));
 }
 
-// out (+)= scale * F'(U)^T w.
+// out (+)= scale * F'(U)^T w, and the face planes add (or null) on top.
 mhd_status rate_vjp(mhd_adjoint* a, const double* const U[6], const double* const w[6], double scale,
-                    int accumulate, double* const out[6]) {
+                    int accumulate, const double* const* add, double* const out[6]) {
     const Domain& D = a->dom;
     AdjScratch& s = a->s;
     k_primitives<<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, cplanes6(U), s.P[0], s.P[1], s.P[2], s.P[3],
@@ -228,21 +223,8 @@ mhd_status rate_vjp(mhd_adjoint* a, const double* const U[6], const double* cons
                                                      planes6(out), s.bc[0], s.bc[1]);
     MHD_TRY(cudaGetLastError());
     k_adj_bfaces<<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, s.bc[0], s.bc[1], s.X[10], s.Y[10], scale,
-                                                      accumulate, out[4], out[5]);
-    MHD_TRY(cudaGetLastError());
-    return MHD_OK;
-}
-
-mhd_status axpby(mhd_adjoint* a, int nplanes, double ca, const double* const* x, double cb,
-                 const double* const* y, double* const* out) {
-    Planes6C X{}, Y{};
-    Planes O{};
-    for (int k = 0; k < nplanes; ++k) {
-        X.f[k] = x[k];
-        Y.f[k] = y ? y[k] : nullptr;
-        O.f[k] = out[k];
-    }
-    k_adj_axpby<<<a->ew_blocks, 256, 0, a->stream>>>(nplanes, a->n, ca, X, cb, Y, O);
+                                                      accumulate, add ? add[0] : nullptr, add ? add[1] : nullptr,
+                                                      out[4], out[5]);
     MHD_TRY(cudaGetLastError());
     return MHD_OK;
 }
@@ -256,58 +238,37 @@ mhd_status adjoint_step(mhd_adjoint* a, const double* const U[6], const Slot& sl
     const double eta = a->eta;
     const double cg = a->dt * a->g, cd = a->dt * a->d;
     const double c1md = a->dt * (1.0 - a->d), c1mg = a->dt * (1.0 - a->g);
-    const int B = a->ew_blocks;
-    const dim3 CG2 = cell_grid(D.nx, D.ny);
+    const dim3 G = adj_grid(a);
+    const int nb = (int)(G.x * G.y);
+    double* const dots = a->dot_partial;  // four terms of dL/deta, nb partial sums each
     cudaStream_t st = a->stream;
     mhd_status r;
-    // final combination: B^{n+1} = A_B + cg * eta * C Jz(B2)
-    k_adj_jz<<<CG2, 256, 0, st>>>(D, s.lam[4], s.lam[5], 1.0, nullptr, 0.0, s.c1);
-    k_adj_jz<<<CG2, 256, 0, st>>>(D, sl.A[4], sl.A[5], 1.0, x2, cg, s.c2);  // Jz(B2)
+    // final combination: B^{n+1} = A_B + cg * eta * C Jz(B2); c2 = Jz(B2), fb = lambda_B2
+    k_adj_resistive<false><<<G, 256, 0, st>>>(D, s.lam[4], s.lam[5], sl.A[4], sl.A[5], x2, cg, cg * eta, s.c2, s.fb[0],
+                                              s.fb[1], nullptr, nullptr, dots);
     MHD_TRY(cudaGetLastError());
-    if ((r = dot_acc(a, s.c1, s.c2, -cg)) != MHD_OK) return r;
-    k_adj_curl<<<CG2, 256, 0, st>>>(D, s.c1, cg * eta, nullptr, nullptr, 0.0, nullptr, nullptr, 0.0,
-                                  s.fb[0], s.fb[1]);  // lambda_B2
-    MHD_TRY(cudaGetLastError());
-    // B2 = A_B + cg S(A_B)
+    // B2 = A_B + cg S(A_B): lambda_A_B
     if ((r = solve(a, s.fb[0], s.fb[1], cg, s.y)) != MHD_OK) return r;
-    k_adj_curl<<<CG2, 256, 0, st>>>(D, s.y, eta, s.lam[4], s.lam[5], 1.0, s.fb[0], s.fb[1], 1.0,
-                                  s.lam[4], s.lam[5]);  // lambda_A_B
+    k_adj_implicit<<<G, 256, 0, st>>>(D, eta, s.y, s.c2, s.fb[0], s.fb[1], s.lam[4], s.lam[5], dots + nb);
     MHD_TRY(cudaGetLastError());
-    if ((r = dot_acc(a, s.y, s.c2, -1.0)) != MHD_OK) return r;
-    // g2 = R(B1) with weight c1mg
-    k_adj_jz<<<CG2, 256, 0, st>>>(D, s.lam[4], s.lam[5], 1.0, nullptr, 0.0, s.c1);
-    k_adj_jz<<<CG2, 256, 0, st>>>(D, sl.T[4], sl.T[5], 1.0, x1, cg, s.c2);  // Jz(B1)
-    MHD_TRY(cudaGetLastError());
-    if ((r = dot_acc(a, s.c1, s.c2, -c1mg)) != MHD_OK) return r;
-    k_adj_curl<<<CG2, 256, 0, st>>>(D, s.c1, c1mg * eta, nullptr, nullptr, 0.0, nullptr, nullptr, 0.0,
-                                  s.fb[0], s.fb[1]);
-    // f2 = F(U1), U1 = (T hydro, B1), weight c1md
-    k_adj_curl<<<CG2, 256, 0, st>>>(D, x1, cg, sl.T[4], sl.T[5], 1.0, nullptr, nullptr, 0.0,
-                                  s.B1[0], s.B1[1]);
+    // g2 = R(B1) with weight c1mg; c2 = Jz(B1); f2 = F(U1), U1 = (T hydro, B1), weight c1md
+    k_adj_resistive<true><<<G, 256, 0, st>>>(D, s.lam[4], s.lam[5], sl.T[4], sl.T[5], x1, cg, c1mg * eta, s.c2, s.fb[0],
+                                             s.fb[1], s.B1[0], s.B1[1], dots + 2 * nb);
     MHD_TRY(cudaGetLastError());
     const double* U1[6] = {sl.T[0], sl.T[1], sl.T[2], sl.T[3], s.B1[0], s.B1[1]};
-    if ((r = rate_vjp(a, U1, s.lam, c1md, 0, s.lamT)) != MHD_OK) return r;
     // lambda_B1 = lamT_B + fb; B1 = T_B + cg S(T_B)
-    {
-        const double* x2p[2] = {s.lamT[4], s.lamT[5]};
-        const double* y2p[2] = {s.fb[0], s.fb[1]};
-        double* o2p[2] = {s.lamT[4], s.lamT[5]};
-        if ((r = axpby(a, 2, 1.0, x2p, 1.0, y2p, o2p)) != MHD_OK) return r;
-    }
+    const double* fb[2] = {s.fb[0], s.fb[1]};
+    if ((r = rate_vjp(a, U1, s.lam, c1md, 0, fb, s.lamT)) != MHD_OK) return r;
     if ((r = solve(a, s.lamT[4], s.lamT[5], cg, s.y)) != MHD_OK) return r;
-    k_adj_curl<<<CG2, 256, 0, st>>>(D, s.y, eta, s.lamT[4], s.lamT[5], 1.0, nullptr, nullptr, 0.0,
-                                  s.lamT[4], s.lamT[5]);
-    MHD_TRY(cudaGetLastError());
-    if ((r = dot_acc(a, s.y, s.c2, -1.0)) != MHD_OK) return r;
     // stage 1: T = U + cg f1, A = U + cd f1 (+ ...): lam = lambda_A + lambda_T + F'(U)^T w
-    {
-        Planes6C lt;
-        for (int k = 0; k < 6; ++k) lt.f[k] = s.lamT[k];
-        k_adj_close<<<B, 256, 0, st>>>(a->n, cd, cg, planes6(s.lam), lt, planes6(s.w));
-        MHD_TRY(cudaGetLastError());
-    }
+    Planes6C lt;
+    for (int k = 0; k < 6; ++k) lt.f[k] = s.lamT[k];
+    k_adj_close<<<G, 256, 0, st>>>(D, eta, s.y, s.c2, cd, cg, planes6(s.lam), lt, planes6(s.w), dots + 3 * nb);
+    MHD_TRY(cudaGetLastError());
+    k_adj_dot_final<<<1, 128, 0, st>>>(dots, nb, DotScales{{-cg, -1.0, -c1mg, -1.0}}, a->geta);
+    MHD_TRY(cudaGetLastError());
     const double* wc[6] = {s.w[0], s.w[1], s.w[2], s.w[3], s.w[4], s.w[5]};
-    return rate_vjp(a, U, wc, 1.0, 1, s.lam);
+    return rate_vjp(a, U, wc, 1.0, 1, nullptr, s.lam);
 }
 
 mhd_status read_status(mhd_adjoint* a) {
@@ -417,8 +378,7 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
     }
     if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
     a->geom = mhd_host::solve_geometry(p->nx, p->ny, a->num_sms);
-    a->ew_blocks = std::max(1, std::min((int)((a->n + 255) / 256), a->num_sms * 8));
-    a->dot_blocks = std::max(1, std::min((int)((a->n + 255) / 256), a->num_sms * 2));
+    const dim3 dot_grid = adj_grid(a);
     // memory: checkpoints, slots, scratch
     const size_t xplanes = 2 * (size_t)(a->recompute_solves ? a->every : a->nsteps);
     const size_t planes = (size_t)a->nseg * 6 + (size_t)a->nslots * kSlotPlanes + xplanes +
@@ -428,7 +388,7 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
         cudaMalloc(&a->status, sizeof(DeviceStatus)) != cudaSuccess ||
         cudaMalloc(&a->sync, sizeof(*a->sync)) != cudaSuccess ||
         cudaMalloc(&a->partials, a->geom.partials() * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&a->dot_partial, (size_t)a->dot_blocks * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&a->dot_partial, (size_t)4 * dot_grid.x * dot_grid.y * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&a->geta, sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&a->host_small, 8 * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
@@ -457,7 +417,6 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
     for (int k = 0; k < 6; ++k) s.w[k] = take();
     s.fb[0] = take();
     s.fb[1] = take();
-    s.c1 = take();
     s.c2 = take();
     s.B1[0] = take();
     s.B1[1] = take();
@@ -603,7 +562,7 @@ mhd_status mhd_adj_rate_vjp(mhd_adjoint* a, const double* const u[6], const doub
     if (!u || !w || !out) return MHD_ERR_INVALID_ARGUMENT;
     for (int k = 0; k < 6; ++k)
         if (!u[k] || !w[k] || !out[k]) return MHD_ERR_INVALID_ARGUMENT;
-    if ((s = rate_vjp(a, u, w, 1.0, 0, out)) != MHD_OK) return s;
+    if ((s = rate_vjp(a, u, w, 1.0, 0, nullptr, out)) != MHD_OK) return s;
     MHD_TRY(cudaStreamSynchronize(a->stream));
     return MHD_OK;
 }
@@ -622,10 +581,9 @@ mhd_status mhd_adj_launch_counts(mhd_adjoint* a, int* forward_step, int* adjoint
     if (!a) return MHD_ERR_INVALID_ARGUMENT;
     // forward: stage 1, solve, stage 2, solve, finalize
     if (forward_step) *forward_step = 5;
-    // adjoint: 4 corner currents, 4 dot products (2 launches each), 5 curls, 2 solves,
-    // 2 explicit-rate VJPs (4 kernels + primitives each), 2 plane combinations; plus the
-    // recomputation of the step's explicit stages (stage 1, stage 2, finalize)
-    if (adjoint_step) *adjoint_step = 4 + 8 + 5 + 2 + 10 + 2 + 3 + (a->recompute_solves ? 2 : 0);
+    // adjoint: 4 resistive passes, their sums, 2 solves, 2 explicit-rate VJPs (4 kernels + primitives each); plus
+    // the recomputation of the step's explicit stages (stage 1, stage 2, finalize)
+    if (adjoint_step) *adjoint_step = 4 + 1 + 2 + 10 + 3 + (a->recompute_solves ? 2 : 0);
     return MHD_OK;
 }
 

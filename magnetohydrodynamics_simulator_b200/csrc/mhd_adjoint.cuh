@@ -31,23 +31,25 @@ struct PrimAdj {
     double rho, vx, vy, p, bx, by;
 };
 
-
 // fast_speed (HLL.hpp:107-122): given the adjoint of c_f, accumulate into w's adjoint and bn's.
 __device__ __forceinline__ void fast_speed_vjp(const Prim& w, double bn, double ac, PrimAdj& aw,
                                                double& abn) {
     const double b2 = w.bx * w.bx + w.by * w.by;
-    const double ir = 1.0 / w.rho;
+    const double ir = rcp_nr(w.rho);
     const double a2 = kGammaGas * w.p * ir;
     const double t2 = b2 * ir;
     const double n2 = bn * bn * ir;
     const double sum = t2 + a2;
     const double term = sum * sum - 4.0 * a2 * n2;
-    const double sq = term > 0.0 ? sqrt(term) : 0.0;
-    const double c = sqrt(0.5 * (sum + sq));
+    // (selected after the root: the branch-free root of a non-positive term is NaN)
+    const bool pos = high_word(term) > 0x03f00000;
+    const double root = sqrt_nr(term);
+    const double h = 0.5 * (sum + (pos ? root : 0.0));  // > 0
     // c = sqrt(h), h = (sum + sq) / 2
-    const double ah = c > 0.0 ? ac * 0.5 / c : 0.0;
+    const double ah = ac * 0.5 * rcp_nr(sqrt_nr(h));
     double asum = 0.5 * ah;
-    const double aterm = sq > 0.0 ? 0.5 * ah * 0.5 / sq : 0.0;
+    const double isq = rcp_nr(root);
+    const double aterm = pos ? 0.25 * ah * isq : 0.0;
     asum += aterm * 2.0 * sum;
     double aa2 = -4.0 * n2 * aterm + asum;
     const double an2 = -4.0 * a2 * aterm;
@@ -147,7 +149,7 @@ __device__ __forceinline__ void hll_vjp(const Prim& L, const Prim& R, const Flux
     }
     const Flux UL = conserved<DIR>(L);
     const Flux UR = conserved<DIR>(R);
-    const double inv = 1.0 / (sR - sL);
+    const double inv = rcp_nr(sR - sL);
     const double sLR = sL * sR;
     Flux F, aFL, aFR, aUR, aUL;
     F.rho = (sR * FL.rho - sL * FR.rho + sLR * (UR.rho - UL.rho)) * inv;
@@ -380,7 +382,7 @@ k_adj_cells(Domain D, CPlanes U, PrimPlanes P, CFaceAdjPlanes X, CFaceAdjPlanes 
         avy += -gm1ap * rho_f * vy;
         abxc += -gm1ap * bxc;
         abyc += -gm1ap * byc;
-        const double ir = 1.0 / rho;
+        const double ir = rcp_nr(rho);
         const double amx = avx * ir;
         const double amy = avy * ir;
         double arho = -(avx * vx + avy * vy) * ir;
@@ -400,7 +402,8 @@ k_adj_cells(Domain D, CPlanes U, PrimPlanes P, CFaceAdjPlanes X, CFaceAdjPlanes 
 static __global__ void __launch_bounds__(256)
 k_adj_bfaces(Domain D, const double* __restrict__ bxc_adj, const double* __restrict__ byc_adj,
              const double* __restrict__ xbn, const double* __restrict__ ybn, double scale,
-             int accumulate, double* __restrict__ out_bx, double* __restrict__ out_by) {
+             int accumulate, const double* __restrict__ add_bx, const double* __restrict__ add_by,
+             double* __restrict__ out_bx, double* __restrict__ out_by) {
     const int nx = D.nx, ny = D.ny;
     for (int j = blockIdx.y; j < ny; j += gridDim.y)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
@@ -409,116 +412,137 @@ k_adj_bfaces(Domain D, const double* __restrict__ bxc_adj, const double* __restr
         const size_t gym = (size_t)wrap(j - 1, ny) * nx + i;
         const double abx = 0.5 * (bxc_adj[g] + bxc_adj[gxm]) + xbn[gxm];
         const double aby = 0.5 * (byc_adj[g] + byc_adj[gym]) + ybn[gym];
-        out_bx[g] = accumulate ? out_bx[g] + scale * abx : scale * abx;
-        out_by[g] = accumulate ? out_by[g] + scale * aby : scale * aby;
+        double vx = accumulate ? out_bx[g] + scale * abx : scale * abx;
+        double vy = accumulate ? out_by[g] + scale * aby : scale * aby;
+        if (add_bx) {  // planes added on top (null: none)
+            vx += add_bx[g];
+            vy += add_by[g];
+        }
+        out_bx[g] = vx;
+        out_by[g] = vy;
     }
 }
 
 // ------------------------------------------------------------------------------------------
 // Linear stencils of the resistive term and plane algebra.
 
-// out = s * Jz(bx, by) + t * L x  (corner plane; x may be null when t == 0).
-static __global__ void __launch_bounds__(256)
-k_adj_jz(Domain D, const double* __restrict__ bx, const double* __restrict__ by, double s,
-         const double* __restrict__ x, double t, double* __restrict__ out) {
-    const int nx = D.nx, ny = D.ny;
-    const double idx = 1.0 / D.dx, idy = 1.0 / D.dy;
-    for (int j = blockIdx.y; j < ny; j += gridDim.y)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
-        const size_t g = (size_t)j * nx + i;
-        const size_t gxm = (size_t)j * nx + wrap(i - 1, nx);
-        const size_t gym = (size_t)wrap(j - 1, ny) * nx + i;
-        double v = s * ((by[g] - by[gxm]) * idx - (bx[g] - bx[gym]) * idy);
-        if (x) {
-            const size_t gxp = (size_t)j * nx + wrap(i + 1, nx);
-            const size_t gyp = (size_t)wrap(j + 1, ny) * nx + i;
-            const double lap = (x[gxp] + x[gxm] - 2.0 * x[g]) * (idx * idx) +
-                               (x[gyp] + x[gym] - 2.0 * x[g]) * (idy * idy);
-            v += t * lap;
-        }
-        out[g] = v;
-    }
-}
+// Each kernel below is one pass that also forms one term of dL/deta: a thread's cells in row order, a block's
+// sum in partial[block] (launch shape adj_grid). They take the place of a corner current, a curl, a dot product
+// and a plane combination at a time: at 1024^2 those were 9-11 us each, most of it launch and tail.
 
-// (out_bx, out_by) = a * (base_bx, base_by) + b * (extra_bx, extra_by) + s * C(E) with
-// C(E) = (-(E(i,j+1) - E(i,j))/dy, (E(i+1,j) - E(i,j))/dx). Null base / extra planes count as 0;
-// out may alias base.
-static __global__ void __launch_bounds__(256)
-k_adj_curl(Domain D, const double* __restrict__ E, double s, const double* base_bx,
-           const double* base_by, double a, const double* extra_bx, const double* extra_by,
-           double b, double* out_bx, double* out_by) {
-    const int nx = D.nx, ny = D.ny;
-    const double idx = 1.0 / D.dx, idy = 1.0 / D.dy;
-    for (int j = blockIdx.y; j < ny; j += gridDim.y)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
-        const size_t g = (size_t)j * nx + i;
-        const size_t gxp = (size_t)j * nx + wrap(i + 1, nx);
-        const size_t gyp = (size_t)wrap(j + 1, ny) * nx + i;
-        double rbx = E ? s * (-(E[gyp] - E[g]) * idy) : 0.0;
-        double rby = E ? s * ((E[gxp] - E[g]) * idx) : 0.0;
-        if (base_bx) { rbx += a * base_bx[g]; rby += a * base_by[g]; }
-        if (extra_bx) { rbx += b * extra_bx[g]; rby += b * extra_by[g]; }
-        out_bx[g] = rbx;
-        out_by[g] = rby;
-    }
-}
-
-// out[k] = a * x[k] + b * y[k] for the planes k < nplanes (y may be null; out may alias x or y).
 struct Planes6C {
     const double* f[6];
 };
-static __global__ void __launch_bounds__(256)
-k_adj_axpby(int nplanes, size_t n, double a, Planes6C x, double b, Planes6C y, Planes out) {
-    for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < n;
-         g += (size_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            if (k < nplanes) {
-                double v = a * x.f[k][g];
-                if (y.f[k]) v += b * y.f[k][g];
-                out.f[k][g] = v;
-            }
-        }
-    }
+
+// Jz(bx, by) at corner (i, j); im, jm: the wrapped column to the left, the row below (offsets).
+__device__ __forceinline__ double adj_jz(const double* __restrict__ bx, const double* __restrict__ by, size_t row, size_t rowm,
+                                         int i, int im, double idx, double idy) {
+    return (by[row + i] - by[row + im]) * idx - (bx[row + i] - bx[rowm + i]) * idy;
 }
 
-// The two plane combinations that close the adjoint step, in one pass over six planes:
-// w = cd * lam + cg * lamT (the explicit-rate adjoint of stage 1) and lam += lamT.
+// Where a resistive term with field B2 = B + t C(x) (x: the solution of the term's solve) meets the adjoint
+// lam: c2 = Jz(B) + t L x = Jz(B2); fb = s C(Jz(lam)); partial sums of Jz(lam) . c2. FIELD: also B2 itself.
+template <bool FIELD>
 static __global__ void __launch_bounds__(256)
-k_adj_close(size_t n, double cd, double cg, Planes lam, Planes6C lamT, Planes w) {
-    for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < n;
-         g += (size_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const double a = lam.f[k][g], t = lamT.f[k][g];
-            w.f[k][g] = cd * a + cg * t;
-            lam.f[k][g] = a + t;
-        }
-    }
-}
-
-// Deterministic dot product: per-block partial sums of a*b, then one block sums them in order
-// and adds scale * total to *acc.
-static __global__ void __launch_bounds__(256)
-k_adj_dot_partial(size_t n, const double* __restrict__ a, const double* __restrict__ b,
-                  double* __restrict__ partial) {
+k_adj_resistive(Domain D, const double* __restrict__ lbx, const double* __restrict__ lby, const double* __restrict__ bx,
+                const double* __restrict__ by, const double* __restrict__ x, double t, double s, double* __restrict__ c2,
+                double* __restrict__ fbx, double* __restrict__ fby, double* __restrict__ b2x, double* __restrict__ b2y,
+                double* __restrict__ partial) {
     __shared__ double red[64];
-    double s[1] = {0.0};
-    for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < n;
-         g += (size_t)gridDim.x * blockDim.x)
-        s[0] += a[g] * b[g];
-    block_sum<256, 1>(s, red);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+    const int nx = D.nx, ny = D.ny;
+    const double idx = 1.0 / D.dx, idy = 1.0 / D.dy;
+    double acc[1] = {0.0};
+    for (int j = blockIdx.y; j < ny; j += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
+        const int im = wrap(i - 1, nx), ip = wrap(i + 1, nx);
+        const size_t row = (size_t)j * nx, rowm = (size_t)wrap(j - 1, ny) * nx, rowp = (size_t)wrap(j + 1, ny) * nx;
+        const size_t g = row + i;
+        const double e = adj_jz(lbx, lby, row, rowm, i, im, idx, idy);
+        const double er = adj_jz(lbx, lby, row, rowm, ip, i, idx, idy);
+        const double eu = adj_jz(lbx, lby, rowp, row, i, im, idx, idy);
+        const double xc = x[g], xr = x[row + ip], xu = x[rowp + i];
+        double v = adj_jz(bx, by, row, rowm, i, im, idx, idy);
+        const double lap = (xr + x[row + im] - 2.0 * xc) * (idx * idx) + (xu + x[rowm + i] - 2.0 * xc) * (idy * idy);
+        v += t * lap;
+        c2[g] = v;
+        fbx[g] = s * (-(eu - e) * idy);
+        fby[g] = s * ((er - e) * idx);
+        if (FIELD) {
+            b2x[g] = t * (-(xu - xc) * idy) + bx[g];
+            b2y[g] = t * ((xr - xc) * idx) + by[g];
+        }
+        acc[0] += e * v;
+    }
+    block_sum<256, 1>(acc, red);
+    if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = acc[0];
 }
 
-// One warp: lane l sums partials l, l+32, ... in order, then a fixed shuffle tree.
-static __global__ void k_adj_dot_final(const double* __restrict__ partial, int nblocks, double scale,
-                                       double* acc) {
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += 32) s += partial[b];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) *acc += scale * s;
+// lam_B += fb + eta C(y), and the partial sums of y . c2.
+static __global__ void __launch_bounds__(256)
+k_adj_implicit(Domain D, double eta, const double* __restrict__ y, const double* __restrict__ c2,
+               const double* __restrict__ fbx, const double* __restrict__ fby, double* __restrict__ lbx,
+               double* __restrict__ lby, double* __restrict__ partial) {
+    __shared__ double red[64];
+    const int nx = D.nx, ny = D.ny;
+    const double idx = 1.0 / D.dx, idy = 1.0 / D.dy;
+    double acc[1] = {0.0};
+    for (int j = blockIdx.y; j < ny; j += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
+        const size_t row = (size_t)j * nx, g = row + i;
+        const double yc = y[g], yr = y[row + wrap(i + 1, nx)], yu = y[(size_t)wrap(j + 1, ny) * nx + i];
+        lbx[g] = eta * (-(yu - yc) * idy) + lbx[g] + fbx[g];
+        lby[g] = eta * ((yr - yc) * idx) + lby[g] + fby[g];
+        acc[0] += yc * c2[g];
+    }
+    block_sum<256, 1>(acc, red);
+    if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = acc[0];
+}
+
+// The end of the adjoint step: lamT_B += eta C(y), the explicit-rate adjoint of stage 1 w = cd lam + cg lamT,
+// lam += lamT, and the partial sums of y . c2.
+static __global__ void __launch_bounds__(256)
+k_adj_close(Domain D, double eta, const double* __restrict__ y, const double* __restrict__ c2, double cd, double cg,
+            Planes lam, Planes6C lamT, Planes w, double* __restrict__ partial) {
+    __shared__ double red[64];
+    const int nx = D.nx, ny = D.ny;
+    const double idx = 1.0 / D.dx, idy = 1.0 / D.dy;
+    double acc[1] = {0.0};
+    for (int j = blockIdx.y; j < ny; j += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x) {
+        const size_t row = (size_t)j * nx, g = row + i;
+        const double yc = y[g], yr = y[row + wrap(i + 1, nx)], yu = y[(size_t)wrap(j + 1, ny) * nx + i];
+        double t[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t[k] = lamT.f[k][g];
+        t[4] = eta * (-(yu - yc) * idy) + t[4];
+        t[5] = eta * ((yr - yc) * idx) + t[5];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const double a = lam.f[k][g];
+            w.f[k][g] = cd * a + cg * t[k];
+            lam.f[k][g] = a + t[k];
+        }
+        acc[0] += yc * c2[g];
+    }
+    block_sum<256, 1>(acc, red);
+    if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = acc[0];
+}
+
+// *acc += sum_k scale[k] * (sum of the kth nblocks partials), one warp a term, in a fixed order.
+struct DotScales {
+    double s[4];
+};
+static __global__ void __launch_bounds__(128)
+k_adj_dot_final(const double* __restrict__ partial, int nblocks, DotScales scale, double* acc) {
+    __shared__ double term[4];
+    const int k = threadIdx.x >> 5, l = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll 8
+    for (int b = l; b < nblocks; b += 32) v += partial[(size_t)k * nblocks + b];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (l == 0) term[k] = scale.s[k] * v;
+    __syncthreads();
+    if (threadIdx.x == 0) *acc += term[0] + term[1] + term[2] + term[3];
 }
 
 }  // namespace mhd
