@@ -33,7 +33,7 @@
 #include <new>
 #include <vector>
 
-#include "mhd_adjoint.cuh"
+#include "mhd_adjoint_sweep.cuh"
 #include "mhd_finalize_sweep.cuh"
 #include "mhd_host_util.h"
 #include "mhd_solve.h"
@@ -44,7 +44,7 @@ using namespace mhd;
 namespace {
 
 constexpr int kSlotPlanes = 14;     // T[6], A[6], Bn[2]
-constexpr int kScratchPlanes = 58;  // adjoint-step and solver scratch (see AdjScratch)
+constexpr int kScratchPlanes = 28;  // adjoint-step and solver scratch (see AdjScratch)
 
 struct Slot {
     double* T[6];
@@ -62,10 +62,6 @@ struct AdjScratch {
     double* y;        // solver solution / adjoint solve
     double* r[2];
     double* p[2];
-    double* P[6];     // primitives of the explicit-rate adjoint
-    double* X[11];    // x-face adjoints
-    double* Y[11];    // y-face adjoints
-    double* bc[2];    // cell-centred B adjoints
 };
 
 }  // namespace
@@ -93,7 +89,7 @@ struct mhd_adjoint {
     double* dot_partial = nullptr;
     double* geta = nullptr;  // device accumulator of dL/deta
     double* host_small = nullptr;
-    SweepGeom sg[2]{}, fg{};
+    SweepGeom sg[2]{}, fg{}, vg{};
     int st_blocks[2]{}, fn_blocks = 0;
     mhd_host::SolveGeom geom;  // implicit solve
     bool have_forward = false;
@@ -197,34 +193,12 @@ dim3 adj_grid(const mhd_adjoint* a) {
     return dim3((unsigned)gx, (unsigned)std::max(1, std::min(a->dom.ny, (a->num_sms * 8 + gx - 1) / gx)));
 }
 
-// out (+)= scale * F'(U)^T w, and the face planes add (or null) on top.
+// out = base + scale * F'(U)^T w; base: six planes of which the first four, or the last two, may be null (= 0).
+// out may be base, but not U or w.
 mhd_status rate_vjp(mhd_adjoint* a, const double* const U[6], const double* const w[6], double scale,
-                    int accumulate, const double* const* add, double* const out[6]) {
-    const Domain& D = a->dom;
-    AdjScratch& s = a->s;
-    k_primitives<<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, cplanes6(U), s.P[0], s.P[1], s.P[2], s.P[3],
-                                                      s.P[4], s.P[5]);
-    MHD_TRY(cudaGetLastError());
-    PrimPlanes P;
-    for (int k = 0; k < 6; ++k) P.f[k] = s.P[k];
-    FaceAdjPlanes X, Y;
-    CFaceAdjPlanes cX, cY;
-    for (int k = 0; k < 11; ++k) {
-        X.f[k] = s.X[k];
-        Y.f[k] = s.Y[k];
-        cX.f[k] = s.X[k];
-        cY.f[k] = s.Y[k];
-    }
-    k_adj_faces<0><<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, P, U[4], U[5], cplanes6(w), X);
-    MHD_TRY(cudaGetLastError());
-    k_adj_faces<1><<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, P, U[4], U[5], cplanes6(w), Y);
-    MHD_TRY(cudaGetLastError());
-    k_adj_cells<<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, cplanes6(U), P, cX, cY, scale, accumulate,
-                                                     planes6(out), s.bc[0], s.bc[1]);
-    MHD_TRY(cudaGetLastError());
-    k_adj_bfaces<<<cell_grid(D.nx, D.ny), 256, 0, a->stream>>>(D, s.bc[0], s.bc[1], s.X[10], s.Y[10], scale,
-                                                      accumulate, add ? add[0] : nullptr, add ? add[1] : nullptr,
-                                                      out[4], out[5]);
+                    const double* const base[6], double* const out[6]) {
+    k_adj_rate_sweep<<<a->vg.nwarps, 32, kAdjSweepSmemBytes, a->stream>>>(a->dom, cplanes6(U), cplanes6(w),
+                                                                         cplanes6(base), scale, planes6(out), a->vg);
     MHD_TRY(cudaGetLastError());
     return MHD_OK;
 }
@@ -257,8 +231,8 @@ mhd_status adjoint_step(mhd_adjoint* a, const double* const U[6], const Slot& sl
     MHD_TRY(cudaGetLastError());
     const double* U1[6] = {sl.T[0], sl.T[1], sl.T[2], sl.T[3], s.B1[0], s.B1[1]};
     // lambda_B1 = lamT_B + fb; B1 = T_B + cg S(T_B)
-    const double* fb[2] = {s.fb[0], s.fb[1]};
-    if ((r = rate_vjp(a, U1, s.lam, c1md, 0, fb, s.lamT)) != MHD_OK) return r;
+    const double* fb[6] = {nullptr, nullptr, nullptr, nullptr, s.fb[0], s.fb[1]};
+    if ((r = rate_vjp(a, U1, s.lam, c1md, fb, s.lamT)) != MHD_OK) return r;
     if ((r = solve(a, s.lamT[4], s.lamT[5], cg, s.y)) != MHD_OK) return r;
     // stage 1: T = U + cg f1, A = U + cd f1 (+ ...): lam = lambda_A + lambda_T + F'(U)^T w
     Planes6C lt;
@@ -267,8 +241,7 @@ mhd_status adjoint_step(mhd_adjoint* a, const double* const U[6], const Slot& sl
     MHD_TRY(cudaGetLastError());
     k_adj_dot_final<<<1, 128, 0, st>>>(dots, nb, DotScales{{-cg, -1.0, -c1mg, -1.0}}, a->geta);
     MHD_TRY(cudaGetLastError());
-    const double* wc[6] = {s.w[0], s.w[1], s.w[2], s.w[3], s.w[4], s.w[5]};
-    return rate_vjp(a, U, wc, 1.0, 1, nullptr, s.lam);
+    return rate_vjp(a, U, s.w, 1.0, s.lam, s.lam);
 }
 
 mhd_status read_status(mhd_adjoint* a) {
@@ -376,6 +349,21 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
         g.nwarps = g.strips_x * g.segs_y;
         a->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;
     }
+    {
+        int occ = 0;
+        if (cudaFuncSetAttribute(k_adj_rate_sweep, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adj_rate_sweep, 32, kAdjSweepSmemBytes) !=
+                cudaSuccess || occ < 1)
+            return fail(MHD_ERR_CUDA);
+        const long long resident = (long long)occ * a->num_sms;
+        SweepGeom& g = a->vg;
+        g.strips_x = (p->nx + AS_OUT - 1) / AS_OUT;
+        const int segs = (int)std::max(1LL, resident / g.strips_x);
+        g.seg_h = std::max(AS_MIN_ROWS, (p->ny + segs - 1) / segs);
+        g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
+        g.nwarps = g.strips_x * g.segs_y;
+    }
     if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
     a->geom = mhd_host::solve_geometry(p->nx, p->ny, a->num_sms);
     const dim3 dot_grid = adj_grid(a);
@@ -425,11 +413,6 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
     s.r[1] = take();
     s.p[0] = take();
     s.p[1] = take();
-    for (int k = 0; k < 6; ++k) s.P[k] = take();
-    for (int k = 0; k < 11; ++k) s.X[k] = take();
-    for (int k = 0; k < 11; ++k) s.Y[k] = take();
-    s.bc[0] = take();
-    s.bc[1] = take();
     if (cudaMemsetAsync(a->pool, 0, planes * a->n * sizeof(double), a->stream) != cudaSuccess ||
         cudaMemsetAsync(a->sync, 0, sizeof(*a->sync), a->stream) != cudaSuccess ||
         cudaMemsetAsync(a->status, 0, sizeof(DeviceStatus), a->stream) != cudaSuccess)
@@ -562,7 +545,11 @@ mhd_status mhd_adj_rate_vjp(mhd_adjoint* a, const double* const u[6], const doub
     if (!u || !w || !out) return MHD_ERR_INVALID_ARGUMENT;
     for (int k = 0; k < 6; ++k)
         if (!u[k] || !w[k] || !out[k]) return MHD_ERR_INVALID_ARGUMENT;
-    if ((s = rate_vjp(a, u, w, 1.0, 0, nullptr, out)) != MHD_OK) return s;
+    // the sweep reads U and w around the cells it writes: through scratch, so that out may be u or w
+    const double* const zero[6] = {};
+    if ((s = rate_vjp(a, u, w, 1.0, zero, a->s.lamT)) != MHD_OK) return s;
+    const double* const r[6] = {a->s.lamT[0], a->s.lamT[1], a->s.lamT[2], a->s.lamT[3], a->s.lamT[4], a->s.lamT[5]};
+    if ((s = copy_planes(a, out, r)) != MHD_OK) return s;
     MHD_TRY(cudaStreamSynchronize(a->stream));
     return MHD_OK;
 }
@@ -581,9 +568,9 @@ mhd_status mhd_adj_launch_counts(mhd_adjoint* a, int* forward_step, int* adjoint
     if (!a) return MHD_ERR_INVALID_ARGUMENT;
     // forward: stage 1, solve, stage 2, solve, finalize
     if (forward_step) *forward_step = 5;
-    // adjoint: 4 resistive passes, their sums, 2 solves, 2 explicit-rate VJPs (4 kernels + primitives each); plus
-    // the recomputation of the step's explicit stages (stage 1, stage 2, finalize)
-    if (adjoint_step) *adjoint_step = 4 + 1 + 2 + 10 + 3 + (a->recompute_solves ? 2 : 0);
+    // adjoint: 4 resistive passes, their sums, 2 solves, 2 explicit-rate VJPs; plus the recomputation of the step's
+    // explicit stages (stage 1, stage 2, finalize)
+    if (adjoint_step) *adjoint_step = 4 + 1 + 2 + 2 + 3 + (a->recompute_solves ? 2 : 0);
     return MHD_OK;
 }
 

@@ -56,15 +56,22 @@ __device__ __forceinline__ double sqrt_nr(double a) {
 #endif
 }
 
-// X * rsqrt(X * r) = sqrt(X / r) for X, r > 0: one third-order step on the reciprocal root instead of a
-// reciprocal and a root.
-__device__ __forceinline__ double sqrt_quotient(double X, double r) {
+// 1 / sqrt(z), z > 0: one third-order step.
+__device__ __forceinline__ double rsqrt_nr(double z) {
 #if defined(__CUDA_ARCH__)
-    const double z = X * r;
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(z));
     const double e = fma(-(z * y), y, 1.0);
-    return X * fma(y * e, fma(0.375, e, 0.5), y);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+#else
+    return 1.0 / sqrt(z);
+#endif
+}
+
+// X * rsqrt(X * r) = sqrt(X / r) for X, r > 0: one reciprocal root instead of a reciprocal and a root.
+__device__ __forceinline__ double sqrt_quotient(double X, double r) {
+#if defined(__CUDA_ARCH__)
+    return X * rsqrt_nr(X * r);
 #else
     return sqrt(X / r);
 #endif
