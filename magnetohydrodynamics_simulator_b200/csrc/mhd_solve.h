@@ -53,10 +53,13 @@ inline SolveGeom solve_geometry(int nx, int ny, int num_sms) {
     const int segs = std::max(1, g.grid * NW / g.strips_x);
     g.seg_h = std::max(4, (ny + segs - 1) / segs);
     g.nwarps = g.strips_x * ((ny + g.seg_h - 1) / g.seg_h);
-    // k_solve: narrow segments of 4 rows or more, four per block until every SM has a block
+    // k_solve: narrow segments of 12 rows, one a warp, until every SM has a block. Spread thinner (4 rows, half
+    // the warps of a block) a solve is 2-6% shorter on a grid of some 60 000 cells, but takes every SM for it: three
+    // contexts stepping 444 x 209, 73 x 914 and 51 x 747 grids on streams of their own then took 250, 562 and 695 us
+    // for 168, 342 and 405 (two, five and seven steps each).
     const int out = mhd::cm_out(mhd::CM_MAXM, 1);
-    const long long nseg = (long long)((nx + out - 1) / out) * ((ny + 3) / 4);
-    g.mgrid = (int)std::max(1LL, std::min((long long)num_sms, (nseg + 3) / 4));
+    const long long nseg = (long long)((nx + out - 1) / out) * ((ny + 11) / 12);
+    g.mgrid = (int)std::max(1LL, std::min((long long)num_sms, (nseg + mhd::CM_NW - 1) / mhd::CM_NW));
     // the largest cluster whose bands have at least one row
     int cs = mhd::CC_MAX;
     while (cs > 1 && ny < cs) cs /= 2;
