@@ -19,6 +19,7 @@
 
 #include "mhd_batch_solve.cuh"
 #include "mhd_host_util.h"
+#include "mhd_state_io.h"
 
 using namespace mhd;
 
@@ -662,6 +663,11 @@ static mhd_status batch_copy_in(mhd_batch* b, int index, const double* const f[6
     for (int k = 0; k < 6; ++k)
         if (!f[k]) return MHD_ERR_INVALID_ARGUMENT;
     const BatchInst& I = b->h_insts[b->parity][index];
+    if (kind == cudaMemcpyDeviceToDevice &&
+        mhd_host::plain_state(f, I.S, b->ncell[index] * sizeof(double), b->device, false)) {
+        b->have_state[index] = 1;
+        return mhd_host::load_state(I.D, f, I.S, b->status + index, b->stream);
+    }
     for (int k = 0; k < 6; ++k)
         MHD_TRY(cudaMemcpyAsync(I.S[k], f[k], b->ncell[index] * sizeof(double), kind, b->stream));
     b->have_state[index] = 1;
@@ -674,6 +680,9 @@ static mhd_status batch_copy_out(mhd_batch* b, int index, double* const f[6], cu
     if (!f) return MHD_ERR_INVALID_ARGUMENT;
     if (!b->have_state[index]) return MHD_ERR_NO_STATE;
     const BatchInst& I = b->h_insts[b->parity][index];
+    if (kind == cudaMemcpyDeviceToDevice &&
+        mhd_host::plain_state(f, I.S, b->ncell[index] * sizeof(double), b->device, true))
+        return mhd_host::store_state(b->ncell[index], I.S, f, b->num_sms, b->stream);
     for (int k = 0; k < 6; ++k) {
         if (!f[k]) continue;
         MHD_TRY(cudaMemcpyAsync(f[k], I.S[k], b->ncell[index] * sizeof(double), kind, b->stream));

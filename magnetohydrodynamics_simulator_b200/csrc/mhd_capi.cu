@@ -20,6 +20,7 @@
 
 #include "../../include/mhd_b200.h"
 #include "mhd_solve.h"
+#include "mhd_state_io.h"
 #include "mhd_snapshot.h"
 #include "mhd_host_util.h"
 #include "mhd_kernels.cuh"
@@ -587,11 +588,15 @@ mhd_status mhd_set_state_device(mhd_context* c, const double* const f[6]) {
     if (s != MHD_OK) return s;
     if ((s = join_transfers(c)) != MHD_OK) return s;
     if (!f) return MHD_ERR_INVALID_ARGUMENT;
-    for (int k = 0; k < 6; ++k) {
+    for (int k = 0; k < 6; ++k)
         if (!f[k]) return MHD_ERR_INVALID_ARGUMENT;
+    if (mhd_host::plain_state(f, c->S, c->n * sizeof(double), c->device, false)) {
+        c->have_state = true;
+        return mhd_host::load_state(c->dom, f, c->S, c->status, c->stream);
+    }
+    for (int k = 0; k < 6; ++k)
         MHD_TRY(cudaMemcpyAsync(c->S[k], f[k], c->n * sizeof(double), cudaMemcpyDeviceToDevice,
                                 c->stream));
-    }
     c->have_state = true;
     return refresh_cfl(c);
 }
@@ -618,6 +623,8 @@ mhd_status mhd_get_state_device(mhd_context* c, double* const f[6]) {
     if (s != MHD_OK) return s;
     if (!f) return MHD_ERR_INVALID_ARGUMENT;
     if (!c->have_state) return MHD_ERR_NO_STATE;
+    if (mhd_host::plain_state(f, c->S, c->n * sizeof(double), c->device, true))
+        return mhd_host::store_state(c->n, c->S, f, c->num_sms, c->stream);
     for (int k = 0; k < 6; ++k) {
         if (!f[k]) continue;
         MHD_TRY(cudaMemcpyAsync(f[k], c->S[k], c->n * sizeof(double), cudaMemcpyDeviceToDevice,
