@@ -21,7 +21,7 @@
 // running error bound (the sums' relative error is far below kCmNoise), and only norms well above
 // it are used. If the residual has not passed the threshold at the last usable k, the ordinary
 // iterations go on from there: r, p and x of an earlier iterate are evaluated from their polynomials
-// (three more passes) and the sweeps of mhd_cg_sweep.cuh go on, in this kernel or in k_cg_sweep launched
+// (three more passes) and the sweeps of mhd_cg_sweep.cuh go on, in this kernel or in the CG kernel launched
 // behind it. With no usable norm, or beyond kCmMaxT, they start from the right-hand side.
 //
 // Bound by instruction issue at two warps a scheduler (FP64 pipe 40%, DRAM 30%), not by DRAM. Measured on
@@ -551,7 +551,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     CgScal s = cg_scalars(a);
     const double t = 2 * (s.cx + s.cy);
     const bool in_range = t >= 1e-30 && t <= kCmMaxT;
-    if (a.start && !in_range) {  // k_cg_sweep, launched next, does all of it
+    if (a.start && !in_range) {  // the CG kernel launched next does all of it
         if (blockIdx.x == 0 && tid == 0) a.start->k = 0;
         return;
     }
@@ -620,7 +620,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
             start.bb = plan.bb;
             start.threshold = plan.threshold;
         }
-        if (a.start) {  // k_cg_sweep, launched next, takes over
+        if (a.start) {  // the CG kernel launched next takes over
             report = false;
             if (blockIdx.x == 0 && tid == 0) *a.start = start;
         } else {
@@ -649,7 +649,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     }
     if (blockIdx.x == 0 && tid == 0) {
         if (report) cg_report(a, res);
-        // solved, or given up: nothing is left for k_cg_sweep
+        // solved, or given up: nothing is left for the CG kernel
         if (a.start && (report || !alive)) a.start->k = -1;
     }
 }

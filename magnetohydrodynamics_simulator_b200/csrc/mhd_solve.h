@@ -3,7 +3,7 @@
 
 #include <algorithm>
 
-#include "mhd_cg_cluster.cuh"
+#include "mhd_cg_band.cuh"
 #include "mhd_cg_moments.cuh"
 #include "mhd_host_util.h"
 
@@ -14,9 +14,10 @@ struct SolveGeom {
     int grid = 0;                             // k_cg_sweep's blocks
     int mgrid = 0;                            // k_solve's blocks
     int cluster = 0;                          // k_cg_cluster's blocks; 0: the grid does not fit a cluster
+    int band = 0;                             // k_cg_band's blocks; 0: the grid does not fit the chip's shared memory
     // doubles of the partial sums of either kernel
     size_t partials() const {
-        return std::max((size_t)2 * grid * 4, (size_t)mgrid * (mhd::CM_NMU + 8));
+        return std::max((size_t)2 * std::max(grid, band) * 4, (size_t)mgrid * (mhd::CM_NMU + 8));
     }
 };
 
@@ -27,8 +28,8 @@ struct SolveSync {
     mhd::CgStart start;
 };
 
-// Once per device: the kernels' shared-memory limits.
-inline mhd_status solve_setup() {
+// Once per device: the kernels' shared-memory limits. (static, as the kernels: every translation unit has its own.)
+static inline mhd_status solve_setup() {
     int occ = 0;
     for (auto k : {mhd::k_cg_sweep<false>, mhd::k_cg_sweep<true>}) {
         MHD_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mhd::kCgRingBytes));
@@ -37,6 +38,8 @@ inline mhd_status solve_setup() {
     }
     MHD_TRY(cudaFuncSetAttribute(mhd::k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(mhd::CC_SMEM_DOUBLES * sizeof(double))));
+    MHD_TRY(cudaFuncSetAttribute(mhd::k_cg_band, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(mhd::CB_SMEM_DOUBLES * sizeof(double))));
     MHD_TRY(cudaFuncSetAttribute(mhd::k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)mhd::kCmSmemBytes));
     MHD_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mhd::k_solve, mhd::CM_NT, mhd::kCmSmemBytes));
@@ -44,7 +47,7 @@ inline mhd_status solve_setup() {
 }
 
 // Both kernels: one wave of co-resident blocks, no more than there are rows of work for their warps.
-inline SolveGeom solve_geometry(int nx, int ny, int num_sms) {
+static inline SolveGeom solve_geometry(int nx, int ny, int num_sms) {
     SolveGeom g;
     constexpr int NW = mhd::CGS_NT / 32;
     g.strips_x = (nx + mhd::CG_W - 1) / mhd::CG_W;
@@ -64,6 +67,7 @@ inline SolveGeom solve_geometry(int nx, int ny, int num_sms) {
     int cs = mhd::CC_MAX;
     while (cs > 1 && ny < cs) cs /= 2;
     g.cluster = mhd::cc_fits(nx, ny, cs) ? cs : 0;
+    g.band = mhd::cb_bands(nx, ny, num_sms);
     return g;
 }
 
@@ -74,14 +78,15 @@ inline double solve_t(double alpha, double dx, double dy) {
 
 // Launch the solve of `a` (its geometry, sync and start are set here). t: solve_t where the host knows
 // alpha, else negative (the step's dt is chosen on the device). Up to kCmMaxT k_solve alone (two passes
-// over the face planes), beyond it k_cg_sweep alone (one sweep per product). Where the host does not
-// know, k_solve comes first and k_cg_sweep behind it finds the solve done, or does it: an idle kernel
-// costs 1 us, the sweeps on k_solve's half as many warps a quarter more time (1024^2: 188 against 150 us).
+// over the face planes), beyond it CG alone: k_cg_band where the chip's shared memory holds the grid, else
+// k_cg_sweep (one sweep per product). Where the host does not know, k_solve comes first and CG behind it
+// finds the solve done, or does it: an idle kernel costs 1 us. (k_cg_band starts from the right-hand side;
+// k_cg_sweep also takes up an iteration that k_solve left.)
 // Grids that fit one cluster take k_cg_cluster, whatever the matrix.
 // field: the right-hand side is a caller's field, not an evolved one. Smooth fields take two to four products,
-// and below 1448^2 as many sweeps are shorter than the two passes, whose length does not depend on them
-// (1024^2: 3 products 66 against 76 us; 2048^2: 198 against 154); in a step there are five or more.
-inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool field, SolveSync* dev,
+// and below 1448^2 as many are shorter than the two passes, whose length does not depend on them
+// (1024^2 with k_cg_sweep: 3 products 66 against 76 us; 2048^2: 198 against 154); in a step there are five or more.
+static inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool field, SolveSync* dev,
                                cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.stream = stream;
@@ -116,7 +121,14 @@ inline mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t,
         cfg.dynamicSmemBytes = mhd::kCmSmemBytes;
         MHD_TRY(cudaLaunchKernelEx(&cfg, mhd::k_solve, a));
     }
-    if (sweep) {
+    if (sweep && g.band) {
+        a.sync = &dev->sync[1];
+        cfg.gridDim = dim3(g.band);
+        cfg.blockDim = dim3(mhd::CB_NT);
+        cfg.dynamicSmemBytes =
+            (size_t)mhd::cb_smem_doubles(a.D.nx, (a.D.ny + g.band - 1) / g.band) * sizeof(double);
+        MHD_TRY(cudaLaunchKernelEx(&cfg, mhd::k_cg_band, a));
+    } else if (sweep) {
         a.sync = &dev->sync[1];
         cfg.gridDim = dim3(g.grid);
         cfg.blockDim = dim3(mhd::CGS_NT);

@@ -106,7 +106,7 @@ inline bool plain_state(const double* const* f, const double* const* s, size_t b
 }
 
 // s = f and its CFL speed into status.
-inline mhd_status load_state(const mhd::Domain& D, const double* const* f, double* const* s, mhd::DeviceStatus* status,
+static inline mhd_status load_state(const mhd::Domain& D, const double* const* f, double* const* s, mhd::DeviceStatus* status,
                              cudaStream_t stream) {
     MHD_TRY(cudaMemsetAsync(&status->smax_bits, 0, sizeof(unsigned long long), stream));
     mhd::CPlanes in;
@@ -120,7 +120,7 @@ inline mhd_status load_state(const mhd::Domain& D, const double* const* f, doubl
     return MHD_OK;
 }
 
-inline mhd_status store_state(size_t n, const double* const* s, double* const* f, int num_sms, cudaStream_t stream) {
+static inline mhd_status store_state(size_t n, const double* const* s, double* const* f, int num_sms, cudaStream_t stream) {
     mhd::CPlanes in;
     mhd::Planes out;
     for (int k = 0; k < 6; ++k) {
