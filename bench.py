@@ -53,11 +53,12 @@ WORKLOAD = "orszag_tang_4096x4096_eta1e-4_cfl0.4"
 
 # Algorithmic bytes per zone of each kernel (compulsory-traffic model of the reference algorithm):
 # stage 1 reads U^n (48), writes the accumulator (48), the predictor (48) and the solve's
-# right-hand side (8) = 152; each CG iteration reads and writes x, r, p = 48; stage 2 reads U1*
+# right-hand side (8) = 152; a solve reads the two face planes for the moments (16) and again for
+# the polynomial (16) and writes x (8) = 40, whatever its products; stage 2 reads U1*
 # (48), E1 (8), the accumulator (48), writes U2* (48) and the right-hand side (8) = 160; finalize
 # reads B2* (16), E2 (8), hydro for the CFL (32), writes B^{n+1} (16) = 72.
-# Per step: 384 + 48 * (k1 + k2) bytes per zone.
-ALG_BYTES = {"stage1": 152.0, "stage2": 160.0, "finalize": 72.0, "cg_per_iter": 48.0}
+# Per step: 384 + 2 * 40 bytes per zone.
+ALG_BYTES = {"stage1": 152.0, "stage2": 160.0, "finalize": 72.0, "cg": 40.0}
 KERNELS = ("stage1", "cg1", "stage2", "cg2", "finalize")
 
 
@@ -399,21 +400,17 @@ def run_gpu_arm(args):
     per_kernel = {}
     for name in KERNELS:
         avg_ms = ksum[name] / steps_rec
-        if name == "cg1":
-            alg = ALG_BYTES["cg_per_iter"] * k1
-        elif name == "cg2":
-            alg = ALG_BYTES["cg_per_iter"] * k2
-        else:
-            alg = ALG_BYTES[name]
+        alg = ALG_BYTES["cg" if name in ("cg1", "cg2") else name]
         gbs = alg * zones / (avg_ms * 1e-3) / 1e9
         per_kernel[name] = {"ms": avg_ms, "alg_bytes_per_zone": alg, "achieved_gbs": gbs,
                             "frac": gbs / peak}
-    # the solver kernel (k_cg_sweep) runs twice per step: its share of the step is both launches
+    # the solver kernel (k_solve) runs twice per step: its share of the step is both launches (each with the idle
+    # launch of the CG kernel behind it)
     solver_ms = per_kernel["cg1"]["ms"] + per_kernel["cg2"]["ms"]
-    solver_gbs = ALG_BYTES["cg_per_iter"] * (k1 + k2) * zones / (solver_ms * 1e-3) / 1e9
+    solver_gbs = 2 * ALG_BYTES["cg"] * zones / (solver_ms * 1e-3) / 1e9
     step_kernels_ms = sum(per_kernel[k]["ms"] for k in KERNELS)
     shares = {"k_stage_sweep<1>": per_kernel["stage1"]["ms"] / step_kernels_ms,
-              "k_cg_sweep": solver_ms / step_kernels_ms,
+              "k_solve": solver_ms / step_kernels_ms,
               "k_stage_sweep<2>": per_kernel["stage2"]["ms"] / step_kernels_ms,
               "k_finalize_sweep": per_kernel["finalize"]["ms"] / step_kernels_ms}
     longest = max(KERNELS, key=lambda k: per_kernel[k]["ms"])
@@ -421,7 +418,7 @@ def run_gpu_arm(args):
     # its measured DRAM bytes per zone and per unit, units per launch)
     funcs = {
         "k_stage_sweep<1>": (ALG_BYTES["stage1"] * zones, per_kernel["stage1"]["ms"], 1, "stage1", 1),
-        "k_cg_sweep": (ALG_BYTES["cg_per_iter"] * (k1 + k2) / 2 * zones, solver_ms / 2, 2, "cg", (k1 + k2) / 2),
+        "k_solve": (ALG_BYTES["cg"] * zones, solver_ms / 2, 2, "cg", 1),
         "k_stage_sweep<2>": (ALG_BYTES["stage2"] * zones, per_kernel["stage2"]["ms"], 1, "stage2", 1),
         "k_finalize_sweep": (ALG_BYTES["finalize"] * zones, per_kernel["finalize"]["ms"], 1, "finalize", 1),
     }
@@ -474,9 +471,9 @@ def run_gpu_arm(args):
                 "traffic": traffic_of(name), "fp64_pipe": fp64_of(name, ms, alg)}
 
     dom = figures(dominant)
-    longest_name = {"stage1": "k_stage_sweep<1>", "cg1": "k_cg_sweep", "stage2": "k_stage_sweep<2>",
-                    "cg2": "k_cg_sweep", "finalize": "k_finalize_sweep"}[longest]
-    step_alg = (384.0 + 48.0 * (k1 + k2)) * zones
+    longest_name = {"stage1": "k_stage_sweep<1>", "cg1": "k_solve", "stage2": "k_stage_sweep<2>",
+                    "cg2": "k_solve", "finalize": "k_finalize_sweep"}[longest]
+    step_alg = (384.0 + 2 * ALG_BYTES["cg"]) * zones
     step_ms = ms_max / args.steps
     roofline = {
         "bound": "hbm", "kernel": dominant,
@@ -487,7 +484,7 @@ def run_gpu_arm(args):
         "longest_launch": figures(longest_name),
         "per_function": {f: figures(f) for f in funcs},
         "shares": shares,
-        "step": {"alg_bytes_per_zone": 384.0 + 48.0 * (k1 + k2),
+        "step": {"alg_bytes_per_zone": 384.0 + 2 * ALG_BYTES["cg"],
                  "achieved": step_alg / (step_ms * 1e-3) / 1e9,
                  "frac": step_alg / (step_ms * 1e-3) / 1e9 / peak},
         "kernels": per_kernel,

@@ -90,11 +90,7 @@ __device__ __forceinline__ int batch_next_item(int* queue) {
     return __shfl_sync(0xffffffffu, it, 0);
 }
 
-// Stage 2 of the batch carries its y slopes in shared memory (as a single context's stage 2 does)
-// and keeps the branchy HLL: the persistent kernel holds an item loop around the sweep, which the
-// branch-free HLL pushes into spills. (Measured on B200 on the 64-instance mixed batch: with the
-// carried values in shared memory, per-face y slopes 7.18 -> 6.97 ms per step, carried slopes
-// 6.93 ms.)
+// Stage 2 of the batch carries its y slopes in shared memory, as a single context's stage 2 does.
 #ifndef MHD_BATCH_YREUSE_2
 #define MHD_BATCH_YREUSE_2 1
 #endif

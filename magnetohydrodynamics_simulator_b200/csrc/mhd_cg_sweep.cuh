@@ -23,6 +23,9 @@
 // fixed order (lane tree, warp order, block order), identically in every block, so every block
 // takes the same decisions and the result is deterministic. Grid-wide waits spin with a
 // wall-clock limit (grid_barrier).
+//
+// This form solves grids too large for the chip's shared memory at t beyond the two-pass form's range, and goes
+// on where the two-pass form's norms end (mhd_cg_moments.cuh).
 #pragma once
 
 #include "mhd_kernels.cuh"

@@ -1,7 +1,9 @@
 // Shared device code of the ARS(2,2,2) IMEX step (reference: solvers.hpp:491-613 of
 // RikibabManos/Magnetohydrodynamics_Simulator), for sm_100a, FP64: parameter blocks, helpers,
 // the bounded grid barrier, the step-coefficient / driver kernel, the finalize kernel and the
-// diagnostics. The explicit stages live in mhd_sweep.cuh, the implicit solve in mhd_cg_sweep.cuh.
+// diagnostics. The explicit stages live in mhd_sweep.cuh, the finalize in mhd_finalize_sweep.cuh, the implicit
+// solve in mhd_cg_cluster.cuh (small grids), mhd_cg_moments.cuh (small t), mhd_cg_band.cuh and mhd_cg_sweep.cuh
+// (the rest); mhd_solve.h chooses.
 //
 // HBM layout: every field is a dense, row-major nx*ny plane of doubles (index j*nx + i), periodic in
 // both directions; there are no ghost cells in device memory -- halos are read with periodic index
@@ -9,7 +11,7 @@
 // left face of cell (i,j), byf(i,j) on its bottom face, and the corner field of the implicit solve
 // at the bottom-left corner.
 //
-// One step is six kernels:
+// One step is six kernels (eight where the device chooses dt and with it the form of the solves):
 //   coeffs     dt (given or CFL), stage weights, matrix coefficient
 //   stage<1>   U^n            -> predictor U1* = U^n + dt*g*f1 and accumulator U^n + dt*d*f1
 //   cg         U1*_B          -> corner field E1 of (I - alpha L) E1 = eta J_z(U1*_B)

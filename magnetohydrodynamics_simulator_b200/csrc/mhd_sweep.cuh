@@ -4,8 +4,8 @@
 // i = c0 - 2 + l (the 2-cell MUSCL halo on each side is covered by lanes 0-1 and 30-31). The warp
 // sweeps the rows of its strip upwards; every quantity that the reference computes on whole
 // planes (solvers.hpp:393-402) is computed here one row at a time, with
-//   * the input rows (and stage 2's E1) copied by cp.async into a per-warp ring of 8 row slots in
-//     shared memory, four rows ahead of their first use, so that no register holds raw input,
+//   * the input rows (and stage 2's E1) copied by cp.async into per-warp rings in shared memory, three
+//     to four rows ahead of their first use, so that no register holds raw input,
 //   * the y-direction stencil of the primitives (rows c-1 .. c+2) held in registers as a rolling
 //     window,
 //   * the x-direction stencil (columns i-1 .. i+2) read from neighbouring lanes by shuffles.
@@ -21,6 +21,11 @@
 //   OUT     hydro rates of row c, B rates of row c-1 (solvers.hpp:253-292) + Butcher weights
 // Lane validity: PRIM lanes 0-31, XFACE lanes 1-29, YFACE lanes 0-30, CORNER lanes 2-30, outputs
 // lanes 2-29; other lanes compute values that are never used.
+//
+// Bound by instruction dispatch: an FP64 instruction holds a sub-partition's dispatch for two cycles, and the
+// FP64 and other instructions of a row take about 90% of it at three warps a sub-partition. Inline reciprocals
+// and roots, the clamped-speed HLL and the packed rings took stage 1 from 0.886 to 0.635 ms and stage 2 from
+// 0.954 to 0.722 ms at 4096^2.
 #pragma once
 
 #include "mhd_kernels.cuh"
@@ -62,17 +67,15 @@ __device__ __forceinline__ double shup(double v, int d) { return __shfl_up_sync(
 __device__ __forceinline__ double shdn(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
 
 // Resident warps per SM: 12 for both stages, i.e. 3 per SM sub-partition, whose 16K registers
-// allow at most 168 per thread (the next step, 16 warps, allows 128 and spills). With the input
-// rows in the shared-memory ring both stages fit 168 registers without spilling.
+// allow at most 168 per thread. 16 warps at 128 registers were slower (0.727 and 0.798 ms at 4096^2 for
+// 0.637 and 0.722), as were 14 (0.739 and 0.825).
 #ifndef MHD_SWEEP_MIN_BLOCKS_1
 #define MHD_SWEEP_MIN_BLOCKS_1 (12 / MHD_SW_WARPS)
 #endif
 #ifndef MHD_SWEEP_MIN_BLOCKS_2
 #define MHD_SWEEP_MIN_BLOCKS_2 (12 / MHD_SW_WARPS)
 #endif
-// Limited slopes formed once per cell (both stages; with the input rows in the shared-memory ring
-// the carried slopes fit the 168 registers: stage 1 at 164, measured on B200 at 4096^2: stage 1
-// 0.966 -> 0.891 ms against forming them per face).
+// Limited slopes formed once per cell in both stages (per face they take two minmods more a cell and direction).
 #ifndef MHD_SWEEP_YREUSE_1
 #define MHD_SWEEP_YREUSE_1 1
 #endif
@@ -86,9 +89,6 @@ __device__ __forceinline__ double shdn(double v, int d) { return __shfl_down_syn
 #define MHD_SWEEP_XREUSE_2 1
 #endif
 
-// Where a sweep finds its planes: in(q) the six input planes, x() the corner field E1 (stage 2),
-// a(q) / b(q) the two output plane sets (stage 1: predictor / accumulator; stage 2: - /
-// accumulator, read and written).
 // A sweep reaches its grid through an accessor PL:
 //   in(q) the six input planes, x() the corner field E1 (stage 2), a(q) / b(q) the two output
 //   plane sets (stage 1: predictor / accumulator; stage 2: - / accumulator, read and written);
