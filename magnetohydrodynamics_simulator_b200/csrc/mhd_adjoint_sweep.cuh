@@ -117,7 +117,7 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             Pbx[3] = (bxf2 + bxr2) / 2.0;
             Pby[3] = (s2[5 * 32] + slot(c + 3)[5 * 32 + lane]) / 2.0;
             double rho = s2[0];
-            Pp[3] = primitives(rho, s2[32], s2[64], s2[96], Pbx[3], Pby[3], Pvx[3], Pvy[3]);
+            Pp[3] = primitives_of<false>(rho, s2[32], s2[64], s2[96], Pbx[3], Pby[3], Pvx[3], Pvy[3]);
             Prho[3] = rho;
         }
         if (c < r0 - AS_PRE_FACE) {

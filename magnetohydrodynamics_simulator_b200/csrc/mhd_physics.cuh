@@ -115,14 +115,28 @@ __device__ __forceinline__ double recon_hi(double fm, double f0, double fp) {
     return f0 + 0.5 * minmod(f0 - fm, fp - f0);
 }
 
+// The straight-line forms (rcp_nr, sqrt_nr and what is built on them) are for values of ordinary size: no products
+// that overflow, no arguments outside the approximations' range. A cell within these limits cannot take them out of
+// it; zero densities, infinities, NaN and values beyond 2^100 (velocity, field) or 2^200 (density, pressure) take the
+// operators' division and root and the reference's own selections instead (ANY).
+constexpr unsigned kOrdinaryHigh = (1023u + 200u) << 20;  // high word of 2^200
+
+__device__ __forceinline__ bool ordinary(double rho, double vx, double vy, double p, double bx, double by) {
+    // none of the four is negative, except a NaN, whose high word is above every number's either way
+    const unsigned a = max((unsigned)high_word(rho), (unsigned)high_word(p));
+    const unsigned b = max((unsigned)high_word(vx * vx + vy * vy), (unsigned)high_word(bx * bx + by * by));
+    return max(a, b) < kOrdinaryHigh;
+}
+
 // Grid.hpp:100-136 computePrimitives for one cell. `rho` is replaced by the floored density;
 // velocities divide by the density as stored (before the floor), as the reference does.
 // Returns the (floored) pressure.
-__device__ __forceinline__ double primitives(double& rho, double mx, double my, double E,
-                                             double bxc, double byc, double& vx, double& vy) {
+template <bool ANY>
+__device__ __forceinline__ double primitives_of(double& rho, double mx, double my, double E,
+                                                double bxc, double byc, double& vx, double& vy) {
     // one reciprocal instead of two divisions (<= 1 ulp from m/rho; the reference's fast-math
     // build is free to do the same)
-    const double ir = rcp_nr(rho);
+    const double ir = ANY ? 1.0 / rho : rcp_nr(rho);
     vx = mx * ir;
     vy = my * ir;
     if (rho < kRhoFloor) rho = kRhoFloor;
@@ -131,6 +145,17 @@ __device__ __forceinline__ double primitives(double& rho, double mx, double my, 
     const double eint = E - kin - mag;
     double p = (kGammaGas - 1) * eint;
     if (p < kPFloor) p = kPFloor;
+    return p;
+}
+// ... of any cell
+__device__ __forceinline__ double primitives(double& rho, double mx, double my, double E,
+                                             double bxc, double byc, double& vx, double& vy) {
+    const double stored = rho;
+    double p = primitives_of<false>(rho, mx, my, E, bxc, byc, vx, vy);
+    if (!ordinary(rho, vx, vy, p, bxc, byc)) {
+        rho = stored;
+        p = primitives_of<true>(rho, mx, my, E, bxc, byc, vx, vy);
+    }
     return p;
 }
 
@@ -236,16 +261,24 @@ __device__ __forceinline__ double corner_ez(double eN, double eS, double eE, dou
 }
 
 // diagnostics.hpp:60-77 fastest signal speed of one cell from its stored primitives.
-__device__ __forceinline__ double cfl_speed(double rho_f, double vx, double vy, double p,
-                                            double bxc, double byc) {
+template <bool ANY>
+__device__ __forceinline__ double cfl_speed_of(double rho_f, double vx, double vy, double p,
+                                               double bxc, double byc) {
     const double r = smax(rho_f, 1e-8);
     const double pr = smax(p, 1e-8);
-    const double ir = rcp_nr(r);
+    const double ir = ANY ? 1.0 / r : rcp_nr(r);
     const double a2 = kGammaGas * pr * ir;
     const double b2 = (bxc * bxc + byc * byc) * ir;
     const double v2 = vx * vx + vy * vy;
+    if constexpr (ANY) return sqrt(a2 + b2) + sqrt(v2);
     const double v = sqrt_nr(v2);
     return sqrt_nr(a2 + b2) + (v2 > 1e-290 ? v : 0.0);
+}
+// ... of any cell: infinite where its speed is (a zero density with momentum, an overflow)
+__device__ __forceinline__ double cfl_speed(double rho_f, double vx, double vy, double p,
+                                            double bxc, double byc) {
+    return ordinary(rho_f, vx, vy, p, bxc, byc) ? cfl_speed_of<false>(rho_f, vx, vy, p, bxc, byc)
+                                                : cfl_speed_of<true>(rho_f, vx, vy, p, bxc, byc);
 }
 
 }  // namespace mhd

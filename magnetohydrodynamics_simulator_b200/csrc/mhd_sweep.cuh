@@ -282,7 +282,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             nbyc = (f2[32 + lane] + fac(c + 3)[32 + lane]) / 2.0;
             double rho = h2[0];
             if (MODE == 2 && rho < kRhoFloor) rho = kRhoFloor;  // floored in place (solvers.hpp:522-523)
-            np = primitives(rho, h2[32], h2[64], h2[96], nbxc, nbyc, nvx, nvy);
+            np = primitives_of<false>(rho, h2[32], h2[64], h2[96], nbxc, nbyc, nvx, nvy);
             nrho = rho;
         }
 #pragma unroll
