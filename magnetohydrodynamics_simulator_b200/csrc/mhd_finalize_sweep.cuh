@@ -121,9 +121,7 @@ __device__ __forceinline__ void finalize_sweep_warp(const FA& f, const StepCoeff
             if (rho < kRhoFloor) f.acc(0)[g] = kRhoFloor;
             const double bxc = (bnx_prev + bnx_right) / 2.0;
             const double byc = (bny_prev + bny) / 2.0;
-            double vx, vy;
-            const double p = primitives(rho, h_cur[1], h_cur[2], h_cur[3], bxc, byc, vx, vy);
-            const double sp = cfl_speed(rho, vx, vy, p, bxc, byc);
+            const double sp = cell_cfl_speed(rho, h_cur[1], h_cur[2], h_cur[3], bxc, byc);
             if (sp > vmax) vmax = sp;
             bad |= !(isfinite(rho) && isfinite(h_cur[1]) && isfinite(h_cur[2]) && isfinite(h_cur[3]) &&
                      isfinite(bnx_prev) && isfinite(bny_prev));

@@ -419,9 +419,7 @@ k_finalize(Domain D, const StepCoeffs* __restrict__ C, Planes acc, const double*
         if (rho < kRhoFloor) acc.f[0][g] = kRhoFloor;
         const double bxc = (bx + s.bxn[n + 1]) / 2.0;
         const double byc = (by + s.byn[n + FN_NW]) / 2.0;
-        double vx, vy;
-        const double p = primitives(rho, mx, my, E, bxc, byc, vx, vy);
-        const double sp = cfl_speed(rho, vx, vy, p, bxc, byc);
+        const double sp = cell_cfl_speed(rho, mx, my, E, bxc, byc);
         if (sp > vmax) vmax = sp;
         bad |= !(isfinite(rho) && isfinite(mx) && isfinite(my) && isfinite(E) && isfinite(bx) &&
                  isfinite(by));
@@ -445,9 +443,8 @@ k_cfl_scan(Domain D, CPlanes u, DeviceStatus* st) {
         const int j = (int)(g / nx), i = (int)(g - (size_t)j * nx);
         const double bxc = (u.f[4][g] + u.f[4][(size_t)j * nx + wrap(i + 1, nx)]) / 2.0;
         const double byc = (u.f[5][g] + u.f[5][(size_t)wrap(j + 1, ny) * nx + i]) / 2.0;
-        double rho = u.f[0][g], vx, vy;
-        const double p = primitives(rho, u.f[1][g], u.f[2][g], u.f[3][g], bxc, byc, vx, vy);
-        vmax = smax(vmax, cfl_speed(rho, vx, vy, p, bxc, byc));
+        double rho = u.f[0][g];
+        vmax = smax(vmax, cell_cfl_speed(rho, u.f[1][g], u.f[2][g], u.f[3][g], bxc, byc));
     }
     vmax = block_max<256>(vmax, red);
     if (threadIdx.x == 0) atomicMax(&st->smax_bits, (unsigned long long)__double_as_longlong(vmax));

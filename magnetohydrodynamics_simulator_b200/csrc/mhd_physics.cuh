@@ -94,25 +94,29 @@ __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b 
 
 // MUSCL.hpp:11-17. The test a * b > 0 by the sign bits: an integer instruction for a product and a
 // comparison of the FP64 pipe. (Where it differs -- a zero, a product that underflows -- the smaller operand
-// is below 1e-154; a NaN operand gives NaN or the other operand.)
+// is below 1e-154.) ANY: the product, for which a NaN makes the slope 0.
+template <bool ANY = false>
 __device__ __forceinline__ double minmod(double a, double b) {
 #if defined(__CUDA_ARCH__)
-    const double s = (fabs(a) < fabs(b)) ? a : b;
-    // (the high word decides: cleared, what is left of s is below 1e-313)
-    return __hiloint2double((__double2hiint(a) ^ __double2hiint(b)) >= 0 ? __double2hiint(s) : 0, __double2loint(s));
-#else
+    if constexpr (!ANY) {
+        const double s = (fabs(a) < fabs(b)) ? a : b;
+        // (the high word decides: cleared, what is left of s is below 1e-313)
+        return __hiloint2double((__double2hiint(a) ^ __double2hiint(b)) >= 0 ? __double2hiint(s) : 0, __double2loint(s));
+    }
+#endif
     if (a * b > 0.0) return (fabs(a) < fabs(b)) ? a : b;
     return 0.0;
-#endif
 }
 
 // MUSCL.hpp:26-47, lower (c - s/2) face value of a cell from (left, centre, right)
+template <bool ANY = false>
 __device__ __forceinline__ double recon_lo(double fm, double f0, double fp) {
-    return f0 - 0.5 * minmod(f0 - fm, fp - f0);
+    return f0 - 0.5 * minmod<ANY>(f0 - fm, fp - f0);
 }
 // upper (c + s/2) face value
+template <bool ANY = false>
 __device__ __forceinline__ double recon_hi(double fm, double f0, double fp) {
-    return f0 + 0.5 * minmod(f0 - fm, fp - f0);
+    return f0 + 0.5 * minmod<ANY>(f0 - fm, fp - f0);
 }
 
 // The straight-line forms (rcp_nr, sqrt_nr and what is built on them) are for values of ordinary size: no products
@@ -162,8 +166,17 @@ __device__ __forceinline__ double primitives(double& rho, double mx, double my, 
 // HLL.hpp:107-122 fast magnetosonic speed, c^2 = (s + sqrt(s^2 - 4 a^2 n^2)) / 2 with s = (gamma p + B^2) / rho,
 // a^2 = gamma p / rho, n^2 = Bn^2 / rho. All terms share 1 / rho, so it is taken once, under the root:
 // c = sqrt(X / rho), X = S + sqrt(S^2 - gamma p Bn^2), S = (gamma p + B^2) / 2.
+// ANY: the quotients first, as the reference forms them (p and B^2 may then be beyond 1e154).
+template <bool ANY = false>
 __device__ __forceinline__ double fast_speed(const Prim& w, double bn) {
     const double b2 = w.bx * w.bx + w.by * w.by;
+    if constexpr (ANY) {
+        const double ir = 1.0 / w.rho;
+        const double a2 = kGammaGas * w.p * ir;
+        const double sum = b2 * ir + a2;
+        const double term = sum * sum - 4.0 * a2 * (bn * bn * ir);
+        return sqrt(0.5 * (sum + sqrt(term > 0.0 ? term : 0.0)));
+    }
     const double gp = kGammaGas * w.p;
     const double S = 0.5 * (gp + b2);
     const double D = fma(S, S, -(gp * (bn * bn)));
@@ -215,15 +228,26 @@ __device__ __forceinline__ Flux conserved(const Prim& w) {
 // HLL.hpp:126-172 (DIR = 0) and :177-218 (DIR = 1). L is the lower/left state. The reference takes F_L where
 // sL >= 0, F_R where sR <= 0 and the average between; with sL and sR clamped to the two sides of 0 the
 // average's own weights give those cases, to rounding: straight-line code without selects per component.
-template <int DIR>
+// ANY: the cases themselves (the side that does not count may be infinite or NaN).
+template <int DIR, bool ANY = false>
 __device__ __forceinline__ Flux hll(const Prim& L, const Prim& R) {
     const Flux FL = phys_flux<DIR>(L);
     const Flux FR = phys_flux<DIR>(R);
-    const double cL = fast_speed(L, DIR == 0 ? L.bx : L.by);
-    const double cR = fast_speed(R, DIR == 0 ? R.bx : R.by);
+    const double cL = fast_speed<ANY>(L, DIR == 0 ? L.bx : L.by);
+    const double cR = fast_speed<ANY>(R, DIR == 0 ? R.bx : R.by);
     const double vL = DIR == 0 ? L.vx : L.vy;
     const double vR = DIR == 0 ? R.vx : R.vy;
     const double mn = smin(vL - cL, vR - cR), mx = smax(vL + cL, vR + cR);
+    if constexpr (ANY) {
+        if (mn >= 0) return FL;
+        if (mx <= 0) return FR;
+        const Flux UL = conserved<DIR>(L);
+        const Flux UR = conserved<DIR>(R);
+        const double inv = 1.0 / (mx - mn), sLR = mn * mx;
+        auto avg = [&](double fl, double fr, double ul, double ur) { return (mx * fl - mn * fr + sLR * (ur - ul)) * inv; };
+        return {avg(FL.rho, FR.rho, UL.rho, UR.rho), avg(FL.mx, FR.mx, UL.mx, UR.mx), avg(FL.my, FR.my, UL.my, UR.my),
+                avg(FL.E, FR.E, UL.E, UR.E), avg(FL.bt, FR.bt, UL.bt, UR.bt)};
+    }
     const double sL = high_word(mn) < 0 ? mn : 0.0, sR = high_word(mx) < 0 ? 0.0 : mx;
     const Flux UL = conserved<DIR>(L);
     const Flux UR = conserved<DIR>(R);
@@ -250,13 +274,14 @@ __device__ __forceinline__ bool ct_average(double v, int mode) {
 }
 
 // solvers.hpp:314-340 corner electric field from the four face fluxes and the corner velocity.
+template <bool ANY = false>
 __device__ __forceinline__ double corner_ez(double eN, double eS, double eE, double eW, double vxc,
                                             double vyc, int mode) {
     double ezy, ezx;
     if (ct_average(vyc, mode)) ezy = 0.5 * (eS + eN);
-    else ezy = (high_word(vyc) > 0) ? eS : eN;
+    else ezy = (ANY ? vyc > 0.0 : high_word(vyc) > 0) ? eS : eN;
     if (ct_average(vxc, mode)) ezx = 0.5 * (eE + eW);
-    else ezx = (high_word(vxc) > 0) ? eW : eE;
+    else ezx = (ANY ? vxc > 0.0 : high_word(vxc) > 0) ? eW : eE;
     return 0.5 * (ezx + ezy);
 }
 
@@ -274,11 +299,19 @@ __device__ __forceinline__ double cfl_speed_of(double rho_f, double vx, double v
     const double v = sqrt_nr(v2);
     return sqrt_nr(a2 + b2) + (v2 > 1e-290 ? v : 0.0);
 }
-// ... of any cell: infinite where its speed is (a zero density with momentum, an overflow)
-__device__ __forceinline__ double cfl_speed(double rho_f, double vx, double vy, double p,
-                                            double bxc, double byc) {
-    return ordinary(rho_f, vx, vy, p, bxc, byc) ? cfl_speed_of<false>(rho_f, vx, vy, p, bxc, byc)
-                                                : cfl_speed_of<true>(rho_f, vx, vy, p, bxc, byc);
+// Both, of any cell, from its conserved values (`rho` is replaced by the floored density); the speed is infinite where
+// it overflows or the density is zero.
+__device__ __forceinline__ double cell_cfl_speed(double& rho, double mx, double my, double E, double bxc, double byc) {
+    const double stored = rho;
+    double vx, vy;
+    double p = primitives_of<false>(rho, mx, my, E, bxc, byc, vx, vy);
+    double speed = cfl_speed_of<false>(rho, vx, vy, p, bxc, byc);
+    if (!ordinary(rho, vx, vy, p, bxc, byc)) {
+        rho = stored;
+        p = primitives_of<true>(rho, mx, my, E, bxc, byc, vx, vy);
+        speed = cfl_speed_of<true>(rho, vx, vy, p, bxc, byc);
+    }
+    return speed;
 }
 
 }  // namespace mhd

@@ -33,9 +33,8 @@ k_state_load(Domain D, CPlanes src, Planes dst, DeviceStatus* st) {
         const double byc = (u[5] + src.f[5][(size_t)wrap(j + 1, ny) * nx + i]) / 2.0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) dst.f[k][g] = u[k];
-        double rho = u[0], vx, vy;
-        const double p = primitives(rho, u[1], u[2], u[3], bxc, byc, vx, vy);
-        vmax = smax(vmax, cfl_speed(rho, vx, vy, p, bxc, byc));
+        double rho = u[0];
+        vmax = smax(vmax, cell_cfl_speed(rho, u[1], u[2], u[3], bxc, byc));
     }
     vmax = block_max<256>(vmax, red);
     if (threadIdx.x == 0) atomicMax(&st->smax_bits, (unsigned long long)__double_as_longlong(vmax));

@@ -585,9 +585,8 @@ k_sub_cfl(Interior v, CPlanes u, unsigned long long* out) {
         const size_t g = at(v, i, j);
         const double bxc = (u.f[4][g] + u.f[4][g + 1]) / 2.0;
         const double byc = (u.f[5][g] + u.f[5][g + v.nxe]) / 2.0;
-        double rho = u.f[0][g], vx, vy;
-        const double p = primitives(rho, u.f[1][g], u.f[2][g], u.f[3][g], bxc, byc, vx, vy);
-        vmax = smax(vmax, cfl_speed(rho, vx, vy, p, bxc, byc));
+        double rho = u.f[0][g];
+        vmax = smax(vmax, cell_cfl_speed(rho, u.f[1][g], u.f[2][g], u.f[3][g], bxc, byc));
         bad |= !(isfinite(u.f[0][g]) && isfinite(u.f[1][g]) && isfinite(u.f[2][g]) &&
                  isfinite(u.f[3][g]) && isfinite(u.f[4][g]) && isfinite(u.f[5][g]));
     }

@@ -146,15 +146,17 @@ struct SwTag {
     static constexpr bool value = V;
 };
 
-// The sweep of one warp over rows [r0, r1) of column strip sx of one grid.
-template <int MODE, class PL, bool kYReuse = (MODE == 1) ? MHD_SWEEP_YREUSE_1 : MHD_SWEEP_YREUSE_2,
-          bool kXReuse = (MODE == 1) ? MHD_SWEEP_XREUSE_1 : MHD_SWEEP_XREUSE_2>
-__device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ C, const PL& pl,
-                                                 int sx, int r0, int r1, double* ring) {
+// The sweep of one warp over rows [r0, r1) of column strip sx of one grid; hydro output from row r0h on.
+// Returns r1 + 1, or the sweep row c at which a cell was not of ordinary size: hydro rows below c and face rows
+// below c - 1 are then written, and nothing of the others. ANY: every cell is. (Asking costs 0.8% of a stage at
+// 4096^2, 0.687 -> 0.692 and 0.782 -> 0.789 ms, and up to 0.6 us of a launch on small grids.)
+template <int MODE, class PL, bool kYReuse, bool kXReuse, bool ANY>
+__device__ __forceinline__ int stage_sweep_rows(const StepCoeffs* __restrict__ C, const PL& pl,
+                                                int sx, int r0, int r1, int r0h, double* ring) {
     const int lane = threadIdx.x & 31;
     const int nx = pl.nx();  // setup only: the loop reads the grid through pl
     const int c0 = sx * SW_OUT;
-    if (r0 >= r1) return;
+    if (r0 >= r1) return r1 + 1;
     // kYReuse / kXReuse: limited slopes formed once per cell (y: carried to the next row; x: shared
     // with the lane on the left), or per face as the reference writes them -- the same operands
     // either way
@@ -234,8 +236,9 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
 #pragma unroll
     for (int r = 0; r < SW_FROWS; ++r) issue_row(cstart - 1 + r);
 
+    bool wild = false;  // this lane met a cell for the sweep of any cell
     // One sweep row; kFaces: with the faces, the corner and the outputs (from row r0 - 1 on).
-    auto row = [&](int c, auto faces) {
+    auto row = [&](int c, auto faces) -> bool {
         constexpr bool kFaces = decltype(faces)::value;
         if constexpr (MODE == 1) cp_async_wait<3>();  // rows up to c+3 have landed
         else cp_async_wait<2>();                       // rows up to c+4 have landed
@@ -282,8 +285,13 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             nbyc = (f2[32 + lane] + fac(c + 3)[32 + lane]) / 2.0;
             double rho = h2[0];
             if (MODE == 2 && rho < kRhoFloor) rho = kRhoFloor;  // floored in place (solvers.hpp:522-523)
-            np = primitives_of<false>(rho, h2[32], h2[64], h2[96], nbxc, nbyc, nvx, nvy);
+            np = primitives_of<ANY>(rho, h2[32], h2[64], h2[96], nbxc, nbyc, nvx, nvy);
             nrho = rho;
+            if constexpr (!ANY) {
+                const unsigned face = max((unsigned)high_word(bxf2) & 0x7fffffffu,
+                                          (unsigned)high_word(f2[32 + lane]) & 0x7fffffffu);
+                wild |= !ordinary(nrho, nvx, nvy, np, nbxc, nbyc) || face >= kOrdinaryHigh;
+            }
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -297,14 +305,14 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
 
         if constexpr (!kFaces) {
             if constexpr (kYReuse) {  // the slopes that the first face row takes over
-                Sy(0) = minmod(Prho[2] - Prho[1], Prho[3] - Prho[2]);
-                Sy(1) = minmod(Pvx[2] - Pvx[1], Pvx[3] - Pvx[2]);
-                Sy(2) = minmod(Pvy[2] - Pvy[1], Pvy[3] - Pvy[2]);
-                Sy(3) = minmod(Pp[2] - Pp[1], Pp[3] - Pp[2]);
-                Sy(4) = minmod(Pbxc[2] - Pbxc[1], Pbxc[3] - Pbxc[2]);
+                Sy(0) = minmod<ANY>(Prho[2] - Prho[1], Prho[3] - Prho[2]);
+                Sy(1) = minmod<ANY>(Pvx[2] - Pvx[1], Pvx[3] - Pvx[2]);
+                Sy(2) = minmod<ANY>(Pvy[2] - Pvy[1], Pvy[3] - Pvy[2]);
+                Sy(3) = minmod<ANY>(Pp[2] - Pp[1], Pp[3] - Pp[2]);
+                Sy(4) = minmod<ANY>(Pbxc[2] - Pbxc[1], Pbxc[3] - Pbxc[2]);
             }
             issue_row(c + 7);
-            return;
+            return false;
         }
         // ---- YFACE: top face of (i, c); D = upper y-extrapolation of row c, U = lower of c+1
         //      (MUSCL.hpp:26-47). With kYReuse each row's limited slope is formed once, when the
@@ -313,11 +321,11 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         {
             Prim Dn, Up;
             if constexpr (kYReuse) {
-                const double s_rho = minmod(Prho[2] - Prho[1], Prho[3] - Prho[2]);
-                const double s_vx = minmod(Pvx[2] - Pvx[1], Pvx[3] - Pvx[2]);
-                const double s_vy = minmod(Pvy[2] - Pvy[1], Pvy[3] - Pvy[2]);
-                const double s_p = minmod(Pp[2] - Pp[1], Pp[3] - Pp[2]);
-                const double s_bx = minmod(Pbxc[2] - Pbxc[1], Pbxc[3] - Pbxc[2]);
+                const double s_rho = minmod<ANY>(Prho[2] - Prho[1], Prho[3] - Prho[2]);
+                const double s_vx = minmod<ANY>(Pvx[2] - Pvx[1], Pvx[3] - Pvx[2]);
+                const double s_vy = minmod<ANY>(Pvy[2] - Pvy[1], Pvy[3] - Pvy[2]);
+                const double s_p = minmod<ANY>(Pp[2] - Pp[1], Pp[3] - Pp[2]);
+                const double s_bx = minmod<ANY>(Pbxc[2] - Pbxc[1], Pbxc[3] - Pbxc[2]);
                 Dn.rho = Prho[1] + 0.5 * Sy(0);
                 Dn.vx = Pvx[1] + 0.5 * Sy(1);
                 Dn.vy = Pvy[1] + 0.5 * Sy(2);
@@ -330,19 +338,19 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
                 Up.bx = Pbxc[2] - 0.5 * s_bx;
                 Sy(0) = s_rho; Sy(1) = s_vx; Sy(2) = s_vy; Sy(3) = s_p; Sy(4) = s_bx;
             } else {
-                Dn.rho = recon_hi(Prho[0], Prho[1], Prho[2]);
-                Dn.vx = recon_hi(Pvx[0], Pvx[1], Pvx[2]);
-                Dn.vy = recon_hi(Pvy[0], Pvy[1], Pvy[2]);
-                Dn.p = recon_hi(Pp[0], Pp[1], Pp[2]);
-                Dn.bx = recon_hi(Pbxc[0], Pbxc[1], Pbxc[2]);
-                Up.rho = recon_lo(Prho[1], Prho[2], Prho[3]);
-                Up.vx = recon_lo(Pvx[1], Pvx[2], Pvx[3]);
-                Up.vy = recon_lo(Pvy[1], Pvy[2], Pvy[3]);
-                Up.p = recon_lo(Pp[1], Pp[2], Pp[3]);
-                Up.bx = recon_lo(Pbxc[1], Pbxc[2], Pbxc[3]);
+                Dn.rho = recon_hi<ANY>(Prho[0], Prho[1], Prho[2]);
+                Dn.vx = recon_hi<ANY>(Pvx[0], Pvx[1], Pvx[2]);
+                Dn.vy = recon_hi<ANY>(Pvy[0], Pvy[1], Pvy[2]);
+                Dn.p = recon_hi<ANY>(Pp[0], Pp[1], Pp[2]);
+                Dn.bx = recon_hi<ANY>(Pbxc[0], Pbxc[1], Pbxc[2]);
+                Up.rho = recon_lo<ANY>(Prho[1], Prho[2], Prho[3]);
+                Up.vx = recon_lo<ANY>(Pvx[1], Pvx[2], Pvx[3]);
+                Up.vy = recon_lo<ANY>(Pvy[1], Pvy[2], Pvy[3]);
+                Up.p = recon_lo<ANY>(Pp[1], Pp[2], Pp[3]);
+                Up.bx = recon_lo<ANY>(Pbxc[1], Pbxc[2], Pbxc[3]);
             }
             Dn.by = Up.by = fac(c + 1)[32 + lane];  // byf of row c+1
-            fy = hll<1>(Dn, Up);
+            fy = hll<1, ANY>(Dn, Up);
         }
         // ---- XFACE: right face of (i, c); L = upper x-extrapolation of column i, R = lower of
         //      i+1. With kXReuse every lane limits its own column's slope once and hands its lower
@@ -354,13 +362,13 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             auto xrecon = [&](double q, double& hi, double& lo_right) {
                 if constexpr (kXReuse) {
                     const double dl = q - shup(q, 1);
-                    const double s = minmod(dl, shdn(dl, 1));
+                    const double s = minmod<ANY>(dl, shdn(dl, 1));
                     hi = q + 0.5 * s;
                     lo_right = shdn(q - 0.5 * s, 1);
                 } else {
                     const double qm = shup(q, 1), qp = shdn(q, 1), qpp = shdn(q, 2);
-                    hi = recon_hi(qm, q, qp);
-                    lo_right = recon_lo(q, qp, qpp);
+                    hi = recon_hi<ANY>(qm, q, qp);
+                    lo_right = recon_lo<ANY>(q, qp, qpp);
                 }
             };
             xrecon(Prho[1], L.rho, R.rho);
@@ -369,7 +377,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             xrecon(Pp[1], L.p, R.p);
             xrecon(Pbyc[0], L.by, R.by);
             L.bx = R.bx = shdn(fac(c)[lane], 1);  // bxf(i+1, c)
-            fx = hll<0>(L, R);
+            fx = hll<0, ANY>(L, R);
         }
         // ---- CORNER (i, c): eN = -Fx^By(i-1, c), eS = -Fx^By(i-1, c-1), eE = Fy^Bx(i, c-1),
         //      eW = Fy^Bx(i-1, c-1); corner velocity = mean of the 4 cells
@@ -381,7 +389,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             const double eW = shup(fy_prev(4), 1);
             const double vxc = 0.25 * (Pvx[1] + shup(Pvx[1], 1) + Pvx[0] + shup(Pvx[0], 1));
             const double vyc = 0.25 * (Pvy[1] + shup(Pvy[1], 1) + Pvy[0] + shup(Pvy[0], 1));
-            ez = corner_ez(eN, eS, eE, eW, vxc, vyc, pl.ct_mode());
+            ez = corner_ez<ANY>(eN, eS, eE, eW, vxc, vyc, pl.ct_mode());
         }
         double jz = 0.0;
         if (MODE == 2) {  // eta*J_z(B1) at corner (i, c) (solvers.hpp:450-461)
@@ -390,6 +398,8 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             const double dBx_dy = (fac(c)[lane] - fac(c - 1)[lane]) * idy;
             jz = pl.eta() * (dBy_dx - dBx_dy);
         }
+        // (part of the outputs' conditions, so that a row stays one stretch of straight-line code)
+        const bool stop = !ANY && __any_sync(0xffffffffu, wild);
         // ---- hydro rates of row c
         {
             double f[4];
@@ -397,7 +407,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
             f[1] = -((fx.mx - shup(fx.mx, 1)) * idx + (fy.mx - fy_prev(1)) * idy);
             f[2] = -((fx.my - shup(fx.my, 1)) * idx + (fy.my - fy_prev(2)) * idy);
             f[3] = -((fx.E - shup(fx.E, 1)) * idx + (fy.E - fy_prev(3)) * idy);
-            if (out_lane && c >= r0 && c < r1) {
+            if (out_lane && !stop && c >= r0h && c < r1) {
                 const size_t g = (size_t)c * pl.nx() + i;
                 if constexpr (MODE == 1) {
                     const double* hc = hyd(c) + lane;
@@ -423,7 +433,7 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
                 g2x = -(jz - jz_prev) * idy;
                 g2y = (shdn(jz_prev, 1) - jz_prev) * idx;
             }
-            if (out_lane && c - 1 >= r0 && c - 1 < r1) {
+            if (out_lane && !stop && c - 1 >= r0 && c - 1 < r1) {
                 const size_t g = (size_t)(c - 1) * pl.nx() + i;
                 if constexpr (MODE == 1) {
                     const double* fp = fac(c - 1);
@@ -448,11 +458,28 @@ __device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ 
         ez_prev = ez;
         jz_prev = jz;
         issue_row(c + 7);  // into the slot of row c-1, no longer read
+        return stop;
     };
-    for (int c = cstart; c < r0 - 1; ++c) row(c, SwTag<false>{});
-    for (int c = r0 - 1; c <= r1; ++c) row(c, SwTag<true>{});
+    int c = cstart;
+    bool stopped = false;
+    for (; c < r0 - 1; ++c) row(c, SwTag<false>{});
+    for (; c <= r1 && !stopped; ++c) stopped = row(c, SwTag<true>{});
     cp_async_wait<0>();  // leave no copy in flight into the ring
+    return stopped ? c - 1 : c;
 }
+
+template <int MODE, class PL, bool kYReuse = (MODE == 1) ? MHD_SWEEP_YREUSE_1 : MHD_SWEEP_YREUSE_2,
+          bool kXReuse = (MODE == 1) ? MHD_SWEEP_XREUSE_1 : MHD_SWEEP_XREUSE_2>
+__device__ __forceinline__ void stage_sweep_warp(const StepCoeffs* __restrict__ C, const PL& pl,
+                                                 int sx, int r0, int r1, double* ring) {
+    const int c = stage_sweep_rows<MODE, PL, kYReuse, kXReuse, false>(C, pl, sx, r0, r1, r0, ring);
+    if (c > r1) return;
+    // the rows left, with cells of any size (inlined: as a function of its own it gave the kernel a stack frame, and
+    // every launch took 1 us longer)
+    __syncwarp();
+    stage_sweep_rows<MODE, PL, true, true, true>(C, pl, sx, max(c - 1, r0), r1, max(c, r0), ring);
+}
+
 
 // Dynamic shared memory of a block of the explicit-stage kernels (their warps' row rings).
 constexpr size_t sweep_smem_bytes(int mode) {

@@ -79,3 +79,101 @@ def test_cfl_and_primitives_of_any_cell(m, shape, cell):
         assert np.array_equal(np.sign(g[np.isinf(w)]), np.sign(w[np.isinf(w)])), name
     ctx.close()
     batch.close()
+
+
+def _modes(rng, nx, ny, amp):
+    x, y = 2 * np.pi * np.arange(nx) / nx, 2 * np.pi * np.arange(ny) / ny
+    f = np.zeros((ny, nx))
+    for kx, ky in ((1, 0), (0, 1), (1, 1), (2, -1)):
+        f += amp * rng.uniform(0.5, 1.0) * np.sin(kx * x[None, :] + ky * y[:, None] + rng.uniform(0, 6))
+    return f
+
+
+def _flow(nx, ny, dx, dy, v0, seed, rho=1.0, v=1.0):
+    """A smooth flow in units of rho and v (pressure and field energy in rho v^2)."""
+    rng = np.random.default_rng(seed)
+    m = [_modes(rng, nx, ny, a) for a in (0.05, 0.03, 0.1, 0.1, 0.2)]
+    r, p, vx, vy, az = 1 + m[0], 0.6 + m[1], v0[0] + m[2], v0[1] + m[3], m[4]
+    bx, by = (np.roll(az, -1, 0) - az) / dy, -(np.roll(az, -1, 1) - az) / dx
+    bxc, byc = 0.5 * (bx + np.roll(bx, -1, 1)), 0.5 * (by + np.roll(by, -1, 0))
+    E = p / (5.0 / 3.0 - 1) + 0.5 * r * (vx * vx + vy * vy) + 0.5 * (bxc * bxc + byc * byc)
+    b = np.sqrt(rho) * v
+    return [np.ascontiguousarray(f) for f in (rho * r, rho * v * r * vx, rho * v * r * vy, rho * v * v * E, b * bx, b * by)]
+
+
+@pytest.mark.parametrize("rho,v", [(1e90, 1e35), (1e200, 1e-25), (1e20, 1e70), (1e70, 1.0)])
+@pytest.mark.parametrize("v0", [(0.0, 0.0), (6.0, 0.2), (-5.0, 6.0)])
+def test_step_in_far_units(m, rho, v, v0):
+    """States whose pressure, field energy or products with the density are beyond what the straight-line fluxes
+    take, but well within the quotients' range: two steps against the oracle, at the single-step tolerance of the
+    parity tests (1e-12 relative L-infinity a field)."""
+    from oracle.oracle import Oracle
+
+    nx, ny = 57, 31
+    dx, dy = 2 * np.pi / nx, 1.4 * np.pi / ny
+    eta = 0.01 * v
+    ic = _flow(nx, ny, dx, dy, v0, 7, rho, v)
+    orc = Oracle(nx, ny, dx, dy, eta)
+    orc.set_state(ic)
+    ctx = m.Context(nx, ny, dx, dy, eta)
+    ctx.set_state(ic)
+    batch = m.Batch([{"nx": nx, "ny": ny, "dx": dx, "dy": dy, "eta": eta}])
+    batch.set_state(0, ic)
+    for _ in range(2):
+        dt = 0.5 * orc.cfl_dt()
+        assert abs(0.5 * ctx.cfl_dt() - dt) <= 1e-13 * dt
+        orc.step(dt)
+        ctx.step(dt)
+        batch.step([dt])
+    assert ctx.synchronize_status() == 0 and batch.synchronize_status()[0] == 0
+    for g, h, w in zip(ctx.get_state(), batch.get_state(0), orc.get_state()):
+        assert np.abs(g - w).max() <= 1e-12 * np.abs(w).max()
+        assert np.abs(h - w).max() <= 1e-12 * np.abs(w).max()
+    ctx.close()
+    batch.close()
+
+
+BAD = {"NaN energy": {3: np.nan}, "infinite energy": {3: np.inf}, "infinite momentum": {1: np.inf},
+       "no density": {0: 0.0, 1: 1.0}, "NaN field": {4: np.nan}}
+
+
+@pytest.mark.parametrize("bad", BAD)
+@pytest.mark.parametrize("at", [(0, 0), (27, 2), (28, 16), (56, 30), (40, 11)])
+@pytest.mark.parametrize("v0", [(0.0, 0.0), (6.0, 0.2), (-5.0, 6.0)])
+def test_one_bad_cell_reaches_the_cells_it_reaches_in_the_oracle(m, at, bad, v0):
+    """An ideal step (eta = 0, its solves give 0) of a state with one such cell, at strip and segment edges: the
+    cells that it makes non-finite are those of the scheme in IEEE operations, the others keep their values."""
+    from oracle.oracle import Oracle
+
+    nx, ny = 57, 31
+    dx, dy = 2 * np.pi / nx, 1.4 * np.pi / ny
+    ic = _flow(nx, ny, dx, dy, v0, 9)
+    dt = 1e-3
+    for k, val in BAD[bad].items():
+        ic[k][at[1], at[0]] = val
+    orc = Oracle(nx, ny, dx, dy, 0.0)
+
+    def rate(u):
+        orc.set_state(u)
+        return orc.explicit_rhs()
+
+    g = m.ars_gamma()
+    d = 1 - 1 / (2 * g)
+    with np.errstate(all="ignore"):
+        f1 = rate(ic)
+        u1 = [u + dt * g * f for u, f in zip(ic, f1)]
+        f2 = rate([np.where(u1[0] < 1e-8, 1e-8, u1[0])] + u1[1:])
+        want = [u + dt * d * a + dt * (1 - d) * b for u, a, b in zip(ic, f1, f2)]
+        # the resistive terms are 0 times the current of a field that may not be finite
+        for b in (u1, want):
+            e = 0.0 * ((b[5] - np.roll(b[5], 1, 1)) - (b[4] - np.roll(b[4], 1, 0)))
+            want[4], want[5] = want[4] - (np.roll(e, -1, 0) - e), want[5] + (np.roll(e, -1, 1) - e)
+    ctx = m.Context(nx, ny, dx, dy, 0.0)
+    ctx.set_state(ic)
+    ctx.step(dt)
+    assert ctx.synchronize_status() == 3  # MHD_ERR_NONFINITE
+    for k, (got, w) in enumerate(zip(ctx.get_state(), want)):
+        fin = np.isfinite(w)
+        assert np.array_equal(np.isfinite(got), fin), (k, np.argwhere(np.isfinite(got) != fin)[:8])
+        assert np.abs(got[fin] - w[fin]).max() <= 1e-12 * max(np.abs(w[fin]).max(), 1.0), k
+    ctx.close()
