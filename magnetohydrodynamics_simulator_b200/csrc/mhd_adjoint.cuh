@@ -71,6 +71,31 @@ __device__ __forceinline__ void fast_speed_vjp(const FaceState& w, const FastSpe
     a.bt += w.bt * aS;
 }
 
+// The speed and its VJP with the quotients first, as the reference forms them: for cells of any size.
+__device__ __forceinline__ double fast_speed_any(const FaceState& w) {
+    const double ir = 1.0 / w.rho;
+    const double a2 = kGammaGas * w.p * ir;
+    const double sum = (w.bn * w.bn + w.bt * w.bt) * ir + a2;
+    const double term = sum * sum - 4.0 * a2 * (w.bn * w.bn * ir);
+    return sqrt(0.5 * (sum + sqrt(term > 0.0 ? term : 0.0)));
+}
+__device__ __forceinline__ void fast_speed_any_vjp(const FaceState& w, double ac, FaceState& a) {
+    const double b2 = w.bn * w.bn + w.bt * w.bt;
+    const double ir = 1.0 / w.rho;
+    const double a2 = kGammaGas * w.p * ir, n2 = w.bn * w.bn * ir;
+    const double sum = b2 * ir + a2;
+    const double term = sum * sum - 4.0 * a2 * n2;
+    const double sq = term > 0.0 ? sqrt(term) : 0.0;
+    const double c = sqrt(0.5 * (sum + sq));
+    const double h = c > 0.0 ? 0.25 * ac / c : 0.0;           // adjoint of sum + sq
+    const double t = sq > 0.0 ? 0.5 * h / sq : 0.0;           // of term
+    const double asum = h + 2.0 * t * sum, aa2 = asum - 4.0 * n2 * t, an2 = -4.0 * a2 * t;
+    a.rho -= (aa2 * kGammaGas * w.p + asum * b2 + an2 * (w.bn * w.bn)) * ir * ir;
+    a.p += aa2 * kGammaGas * ir;
+    a.bn += 2.0 * w.bn * (asum + an2) * ir;
+    a.bt += 2.0 * w.bt * asum * ir;
+}
+
 // One side's f.F and f.U (less the terms in bn alone, which cancel between the sides), and what the VJP shares.
 struct FaceSide {
     double K, Mn, Mt, G, hp, phi, ups;
@@ -104,16 +129,37 @@ __device__ __forceinline__ FaceState face_side_vjp(const FaceState& w, const Flu
 }
 
 // L, R: lower and upper state; f: the flux adjoint. The normal field enters both states: its adjoint is the sum of
-// both sides' bn. Selections (HLL.hpp:139-141: std::min, std::max) as in the forward.
+// both sides' bn. Selections (HLL.hpp:139-141: std::min, std::max) as in the forward. ANY: for cells of any size, with
+// the one-sided cases as the forward has them there.
+template <bool ANY>
 __device__ __forceinline__ void hll_vjp(const FaceState& L, const FaceState& R, const FluxAdj& f, FaceState& aL,
                                         FaceState& aR) {
-    const FastSpeed cL = fast_speed_parts(L), cR = fast_speed_parts(R);
+    FastSpeed cL, cR;
+    if constexpr (ANY) {
+        cL.c = fast_speed_any(L);
+        cR.c = fast_speed_any(R);
+    } else {
+        cL = fast_speed_parts(L);
+        cR = fast_speed_parts(R);
+    }
     const FaceSide l = face_side(L, f), r = face_side(R, f);
     const double mnL = L.vn - cL.c, mnR = R.vn - cR.c, mxL = L.vn + cL.c, mxR = R.vn + cR.c;
     const bool lowR = mnR < mnL, highR = mxL < mxR;
     const double mn = lowR ? mnR : mnL, mx = highR ? mxR : mxL;
+    if constexpr (ANY) {
+        if (mn >= 0.0) {
+            aL = face_side_vjp(L, f, l, 0.0, 1.0);
+            aR = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            return;
+        }
+        if (mx <= 0.0) {
+            aL = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            aR = face_side_vjp(R, f, r, 0.0, 1.0);
+            return;
+        }
+    }
     const double sL = mn < 0.0 ? mn : 0.0, sR = mx > 0.0 ? mx : 0.0;
-    const double inv = rcp_nr(sR - sL);
+    const double inv = ANY ? 1.0 / (sR - sL) : rcp_nr(sR - sL);
     const double a = sR * inv, b = sL * inv;
     const double X = r.phi - l.phi, Y = r.ups - l.ups;
     const double asR = mx > 0.0 ? (inv * b) * fma(-sL, Y, X) : 0.0;
@@ -123,8 +169,13 @@ __device__ __forceinline__ void hll_vjp(const FaceState& L, const FaceState& R, 
     const double lL = lowR ? 0.0 : asL, lR = lowR ? asL : 0.0, hL = highR ? 0.0 : asR, hR = highR ? asR : 0.0;
     aL.vn += lL + hL;
     aR.vn += lR + hR;
-    fast_speed_vjp(L, cL, hL - lL, aL);
-    fast_speed_vjp(R, cR, hR - lR, aR);
+    if constexpr (ANY) {
+        fast_speed_any_vjp(L, hL - lL, aL);
+        fast_speed_any_vjp(R, hR - lR, aR);
+    } else {
+        fast_speed_vjp(L, cL, hL - lL, aL);
+        fast_speed_vjp(R, cR, hR - lR, aR);
+    }
 }
 
 // Which operand minmod(a, b) returned (MUSCL.hpp:11-17): 1 = a, 2 = b, 0 = none.

@@ -36,19 +36,13 @@ constexpr int AS_PRE = 6;             // ... and the primitives this many
 // gradient; 6 sweeps half the extra rows of 3.
 constexpr int AS_MIN_ROWS = 6;
 
-static __global__ void __launch_bounds__(32, 8)
-k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Planes out, SweepGeom G) {
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double as_ring_mem[];
-#else
-    static double as_ring_mem[AS_ROWS * AS_SLOT + AS_CARRY];
-#endif
-    double* const ring = as_ring_mem;
+// The sweep of output rows [r0, r1) of strip sx. Returns r1 + 1, or the sweep row c at which a cell was not of ordinary
+// size: output rows below c - 1 are then written, and nothing of the others. ANY: every cell is.
+template <bool ANY>
+__device__ __forceinline__ int adj_rate_rows(const Domain& D, const CPlanes& U, const CPlanes& w, const CPlanes& base,
+                                             double scale, const Planes& out, int sx, int r0, int r1, double* ring) {
     double* const carry = ring + AS_ROWS * AS_SLOT + (threadIdx.x & 31);
     const int lane = threadIdx.x & 31;
-    const int sx = blockIdx.x % G.strips_x, sy = blockIdx.x / G.strips_x;
-    const int r0 = sy * G.seg_h, r1 = min(r0 + G.seg_h, D.ny);
-    if (r0 >= r1) return;
     const int nx = D.nx;
     const int i = sx * AS_OUT - 4 + lane;
     const int iw = wrap(i, nx), iw_r = wrap(i + 1, nx);
@@ -89,7 +83,9 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
 #pragma unroll
     for (int r = 2; r < AS_ROWS - 1; ++r) issue_row(cstart + r);
 
-    for (int c = cstart; c <= r1; ++c) {
+    bool wild = false;  // this lane met a cell for the sweep of any cell
+    int c = cstart;
+    for (; c <= r1; ++c) {
         cp_async_wait<3>();  // rows up to c+3 have landed
         double ob[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         const bool out_row = out_lane && c - 1 >= r0;
@@ -117,8 +113,12 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             Pbx[3] = (bxf2 + bxr2) / 2.0;
             Pby[3] = (s2[5 * 32] + slot(c + 3)[5 * 32 + lane]) / 2.0;
             double rho = s2[0];
-            Pp[3] = primitives_of<false>(rho, s2[32], s2[64], s2[96], Pbx[3], Pby[3], Pvx[3], Pvy[3]);
+            Pp[3] = primitives_of<ANY>(rho, s2[32], s2[64], s2[96], Pbx[3], Pby[3], Pvx[3], Pvy[3]);
             Prho[3] = rho;
+            if constexpr (!ANY) {
+                const unsigned face = max((unsigned)high_word(bxf2) & 0x7fffffffu, (unsigned)high_word(s2[5 * 32]) & 0x7fffffffu);
+                wild |= !ordinary(rho, Pvx[3], Pvy[3], Pp[3], Pbx[3], Pby[3]) || face >= kOrdinaryHigh;
+            }
         }
         if (c < r0 - AS_PRE_FACE) {
             issue_row(c + AS_ROWS - 1);
@@ -148,7 +148,7 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             auto recon = [&](double q, int k, double& hi, double& lo_right) {
                 const double dl = q - up(q);
                 const double dr = dn(dl);
-                const double s = minmod(dl, dr);
+                const double s = minmod<ANY>(dl, dr);
                 hi = q + 0.5 * s;
                 lo_right = dn(q - 0.5 * s);
                 br |= minmod_branch(dl, dr) << (2 * k);
@@ -162,7 +162,7 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             const FluxAdj f = {(dn(w0[0]) - w0[0]) * idx, (dn(w0[32]) - w0[32]) * idx, (dn(w0[64]) - w0[64]) * idx,
                                (dn(w0[96]) - w0[96]) * idx, xbt};
             FaceState aL, aR;
-            hll_vjp(L, R, f, aL, aR);
+            hll_vjp<ANY>(L, R, f, aL, aR);
             xbn = aL.bn + aR.bn;
             auto gather = [&](int k, double hi, double lo_right) {
                 const double lo = up(lo_right);
@@ -183,8 +183,8 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
         {
             FaceState Dn, Up;
             auto recon = [](const double (&q)[4], double& hi, double& lo_up) {
-                hi = recon_hi(q[0], q[1], q[2]);
-                lo_up = recon_lo(q[1], q[2], q[3]);
+                hi = recon_hi<ANY>(q[0], q[1], q[2]);
+                lo_up = recon_lo<ANY>(q[1], q[2], q[3]);
             };
             recon(Prho, Dn.rho, Up.rho);
             recon(Pvx, Dn.vt, Up.vt);
@@ -195,7 +195,7 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             const FluxAdj f = {(w1[0] - w0[0]) * idy, (w1[64] - w0[64]) * idy, (w1[32] - w0[32]) * idy,
                                (w1[96] - w0[96]) * idy, ybt};
             FaceState aD, aU;
-            hll_vjp(Dn, Up, f, aD, aU);
+            hll_vjp<ANY>(Dn, Up, f, aD, aU);
             ybn = aD.bn + aU.bn;
             auto gather = [&](int k, const double (&q)[4], double hi, double lo_up) {
                 const double as = 0.5 * (hi - Lo(k));
@@ -216,6 +216,7 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             for (int k = 0; k < 4; ++k) Acc[k] += ax[k];
             Acc[5] = ax[4];
         }
+        const bool stop = !ANY && __any_sync(0xffffffffu, wild);
         // ---- OUT row c-1: primitive -> conserved (Grid.hpp:100-136): vx = mx/rho, vy = my/rho (density as stored),
         //      rho_f = max(rho, floor), p = max((gamma-1)(E - rho_f v^2/2 - |Bc|^2/2), floor)
         {
@@ -229,13 +230,13 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
             const double avy = a[2] - gm1ap * rho_f * vy;
             const double abxc = a[4] - gm1ap * bxc;
             const double abyc = a[5] - gm1ap * byc;
-            const double ir = rcp_nr(rho);
+            const double ir = ANY ? 1.0 / rho : rcp_nr(rho);
             double arho = -(avx * vx + avy * vy) * ir;
             if (!(rho < kRhoFloor)) arho += arho_f;
             // bxc(i) = (bxf(i) + bxf(i+1))/2, and bxf(i) is the normal field of x face i-1
             const double abx = 0.5 * (abxc + up(abxc)) + up(xbn1);
             const double aby = 0.5 * (abyc + abyc_prev) + ybn2;
-            if (out_row) {
+            if (out_row && !stop) {
                 out.f[0][g] = ob[0] + scale * arho;
                 out.f[1][g] = ob[1] + scale * (avx * ir);
                 out.f[2][g] = ob[2] + scale * (avy * ir);
@@ -249,8 +250,26 @@ k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Pla
         ybn1 = ybn;
         xbn1 = xbn;
         issue_row(c + AS_ROWS - 1);  // into the slot of row c-1, no longer read
+        if (stop) break;
     }
     cp_async_wait<0>();  // leave no copy in flight into the ring
+    return c;
+}
+
+static __global__ void __launch_bounds__(32, 8)
+k_adj_rate_sweep(Domain D, CPlanes U, CPlanes w, CPlanes base, double scale, Planes out, SweepGeom G) {
+#if defined(__CUDA_ARCH__)
+    extern __shared__ __align__(16) double as_ring_mem[];
+#else
+    static double as_ring_mem[AS_ROWS * AS_SLOT + AS_CARRY];
+#endif
+    const int sx = blockIdx.x % G.strips_x, sy = blockIdx.x / G.strips_x;
+    const int r0 = sy * G.seg_h, r1 = min(r0 + G.seg_h, D.ny);
+    if (r0 >= r1) return;
+    const int c = adj_rate_rows<false>(D, U, w, base, scale, out, sx, r0, r1, as_ring_mem);
+    if (c > r1) return;
+    __syncwarp();
+    adj_rate_rows<true>(D, U, w, base, scale, out, sx, max(c - 1, r0), r1, as_ring_mem);  // (inlined: no stack frame)
 }
 
 }  // namespace mhd

@@ -177,3 +177,33 @@ def test_one_bad_cell_reaches_the_cells_it_reaches_in_the_oracle(m, at, bad, v0)
         assert np.array_equal(np.isfinite(got), fin), (k, np.argwhere(np.isfinite(got) != fin)[:8])
         assert np.abs(got[fin] - w[fin]).max() <= 1e-12 * max(np.abs(w[fin]).max(), 1.0), k
     ctx.close()
+
+
+@pytest.mark.parametrize("rho,v", [(1e90, 1e35), (1e200, 1e-25), (1e20, 1e70), (1.0, 1.0)])
+@pytest.mark.parametrize("v0", [(0.0, 0.0), (6.0, 0.2), (-5.0, 6.0)])
+def test_rate_vjp_in_far_units(m, rho, v, v0):
+    """The explicit rate's VJP of such states against PyTorch autograd through the restated rate, at the suite's
+    bound for these quantities (1e-9 relative a field)."""
+    import torch
+
+    from oracle import torch_step as ts
+
+    nx, ny = 53, 17
+    dx, dy = 2 * np.pi / nx, 1.4 * np.pi / ny
+    U = torch.tensor(np.stack(_flow(nx, ny, dx, dy, v0, 7, rho, v)))
+    # an adjoint in the inverse units of the rates, so that every rate counts alike
+    unit = torch.tensor([rho, rho * v, rho * v, rho * v * v, np.sqrt(rho) * v, np.sqrt(rho) * v], dtype=torch.float64)
+    w = torch.randn(6, ny, nx, generator=torch.Generator().manual_seed(5), dtype=torch.float64) / unit[:, None, None]
+    Ut = [U[k].clone().requires_grad_(True) for k in range(6)]
+    want = torch.autograd.grad(ts.explicit_rhs(Ut, dx, dy), Ut, grad_outputs=list(w))
+    assert all(torch.isfinite(t).all() for t in want)
+    adj = m.Adjoint(nx, ny, dx, dy, 1e-2, 1e-3, 1)
+    u_d, w_d = U.cuda().contiguous(), w.cuda().contiguous()
+    out = torch.empty_like(u_d)
+    torch.cuda.synchronize()
+    adj.rate_vjp([u_d[k].data_ptr() for k in range(6)], [w_d[k].data_ptr() for k in range(6)],
+                 [out[k].data_ptr() for k in range(6)])
+    for k in range(6):
+        err = float((out[k].cpu() - want[k]).abs().max() / want[k].abs().max())
+        assert err <= 1e-9, (k, err)
+    adj.close()
