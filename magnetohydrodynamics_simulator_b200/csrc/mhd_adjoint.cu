@@ -364,8 +364,8 @@ mhd_status mhd_adj_create_ex(const mhd_params* p, double dt, int nsteps, int che
         g.segs_y = (p->ny + g.seg_h - 1) / g.seg_h;
         g.nwarps = g.strips_x * g.segs_y;
     }
-    if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
     a->geom = mhd_host::solve_geometry(p->nx, p->ny, a->num_sms);
+    if (mhd_host::solve_setup(&a->geom) != MHD_OK) return fail(MHD_ERR_CUDA);
     const dim3 dot_grid = adj_grid(a);
     // memory: checkpoints, slots, scratch
     const size_t xplanes = 2 * (size_t)(a->recompute_solves ? a->every : a->nsteps);

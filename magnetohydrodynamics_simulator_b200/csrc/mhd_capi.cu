@@ -390,8 +390,8 @@ mhd_status mhd_create(const mhd_params* p, void* stream, mhd_context** out) {
         g.nwarps = g.strips_x * g.segs_y;
         c->fn_blocks = (g.nwarps + FS_WARPS - 1) / FS_WARPS;
     }
-    if (mhd_host::solve_setup() != MHD_OK) return fail(MHD_ERR_CUDA);
     c->solve = mhd_host::solve_geometry(p->nx, p->ny, c->num_sms);
+    if (mhd_host::solve_setup(&c->solve) != MHD_OK) return fail(MHD_ERR_CUDA);
     c->divb_blocks = std::max(1, std::min((int)((c->n + 255) / 256), c->num_sms * 4));
     // memory
     if (cudaMalloc(&c->pool, (size_t)kPlanes * c->n * sizeof(double)) != cudaSuccess) {
@@ -998,7 +998,7 @@ mhd_status noalloc_setup(int dev, NoAllocDevice** out) {
         MHD_TRY(cudaGetSymbolAddress(&addr, g_noalloc_scratch));
         int sms = 0;
         MHD_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const mhd_status s = mhd_host::solve_setup();
+        const mhd_status s = mhd_host::solve_setup(nullptr);
         if (s != MHD_OK) return s;
         d.scratch = static_cast<double*>(addr);
         // one block per SM, as a context launches the solver

@@ -242,30 +242,4 @@ __device__ __forceinline__ bool cb_solve(const CgSweepArgs& a, double* smem, CbS
     return true;
 }
 
-// a.start: behind k_solve, which says there whether anything is left to do.
-static __global__ void __launch_bounds__(CB_NT, 1)
-k_cg_band(const __grid_constant__ CgSweepArgs a) {
-    __shared__ CbShared sh;
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double cb_mem[];
-#else
-    static double cb_mem[CB_SMEM_DOUBLES];
-#endif
-    if (a.start && a.start->k < 0) return;
-    unsigned long long target = barrier_base(a.sync);
-    const unsigned long long deadline = global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
-    auto barrier = [&]() -> bool {
-        if (grid_barrier(a.sync, target, deadline, &sh.flag)) return true;
-        if (threadIdx.x == 0) atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
-        return false;
-    };
-    const int Rmax = (a.D.ny + (int)gridDim.x - 1) / (int)gridDim.x;
-    const long long runs = (long long)a.D.nx * ((Rmax + CB_V - 1) / CB_V);
-    CgResult res{};
-    const bool ok = runs <= CB_NT ? cb_solve<1>(a, cb_mem, &sh, barrier, res)
-                    : runs <= 2 * CB_NT ? cb_solve<2>(a, cb_mem, &sh, barrier, res)
-                                        : cb_solve<CB_ITEMS>(a, cb_mem, &sh, barrier, res);
-    if (ok && blockIdx.x == 0 && threadIdx.x == 0) cg_report(a, res);
-}
-
 }  // namespace mhd

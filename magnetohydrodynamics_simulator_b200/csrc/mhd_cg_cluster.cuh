@@ -222,22 +222,4 @@ __device__ __forceinline__ bool cc_solve_any(const Domain& D, int blocks, double
     return cc_solve<4, CC_ITEMS>(D, alpha_m, bxf, byf, x, tol, max_iters, deadline, smem, tab, res);
 }
 
-static __global__ void __launch_bounds__(CC_NT, 1)
-k_cg_cluster(const __grid_constant__ CgSweepArgs a) {
-    __shared__ CcTable tab;
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double cc_mem[];
-#else
-    static double cc_mem[CC_SMEM_DOUBLES];
-#endif
-    const unsigned long long deadline = global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
-    CgResult res{};
-    const bool ok = cc_solve_any(a.D, gridDim.x, a.C->alpha, a.bxf, a.byf, a.x, a.tol, a.max_iters, deadline, cc_mem, &tab, res);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (ok) cg_report(a, res);
-        else atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
-    }
-    cooperative_groups::this_cluster().sync();  // no block leaves while another may write into its shared memory
-}
-
 }  // namespace mhd

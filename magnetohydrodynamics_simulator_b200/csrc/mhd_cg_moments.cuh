@@ -540,118 +540,4 @@ __device__ __forceinline__ void cm_pass2_any(const CmGeom& g, int deg, int wfirs
     else cm_pass2<CM_MAXM - 1, CM_C>(g, wfirst, warps, q, out);
 }
 
-static __global__ void __launch_bounds__(CM_NT, 1)
-k_solve(const __grid_constant__ CgSweepArgs a) {
-    __shared__ double red[CM_NW][CM_NMU];
-    __shared__ double mu[32];
-    __shared__ double scal[8];
-    __shared__ CmPlan plan;
-    __shared__ int sflag;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    CgScal s = cg_scalars(a);
-    const double t = 2 * (s.cx + s.cy);
-    const bool in_range = t >= 1e-30 && t <= kCmMaxT;
-    if (a.start && !in_range) {  // the CG kernel launched next does all of it
-        if (blockIdx.x == 0 && tid == 0) a.start->k = 0;
-        return;
-    }
-    const int G = gridDim.x, warps = G * CM_NW;
-    // consecutive segments go to different SMs, so that few of them spread out
-    const int wfirst = wid * G + blockIdx.x;
-    unsigned long long target = barrier_base(a.sync);
-    const unsigned long long deadline = global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
-    CmGeom g;
-    g.nx = a.D.nx;
-    g.ny = a.D.ny;
-    g.ratio = a.D.dx / a.D.dy;
-    g.ax = s.cx / t;
-    g.ay = s.cy / t;
-    g.bxf = a.bxf;
-    g.byf = a.byf;
-    const double scale = a.D.eta / a.D.dx;
-    bool alive = true;
-    auto barrier = [&]() {
-        if (alive && !grid_barrier(a.sync, target, deadline, &sflag)) {
-            alive = false;
-            // (any block: one that gives up leaves its part of x unwritten)
-            if (tid == 0) atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
-        }
-        return alive;
-    };
-    int mode = kCmScratch;
-    if (in_range) {
-        const int M = cm_levels(t);
-        if (M == 5) cm_pass1_any<5>(g, wfirst, warps, a.partials, red);
-        else if (M == 7) cm_pass1_any<7>(g, wfirst, warps, a.partials, red);
-        else cm_pass1_any<CM_MAXM>(g, wfirst, warps, a.partials, red);
-        if (barrier()) {
-            // every block adds the blocks' partials in the same order
-            if (tid < 32) mu[tid] = 0.0;
-            __syncthreads();
-            for (int v = wid; v <= 2 * M; v += CM_NW) {
-                double x = 0.0;
-#pragma unroll 5
-                for (int b = lane; b < G; b += 32) x += __ldcg(&a.partials[(size_t)v * G + b]);
-                for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                if (lane == 0) mu[v] = x * (scale * scale);
-            }
-            __syncthreads();
-            if (wid == 0) cm_plan(mu[lane], M, t, s.diag, scale, a.tol, a.max_iters, &plan);
-            __syncthreads();
-            mode = plan.mode;
-            if (mode == kCmDone || mode == kCmCapped || mode == kCmContinue)
-                cm_pass2_any(g, plan.k - 1, wfirst, warps, plan.q, a.x);
-        }
-    }
-    CgResult res{};
-    bool report = alive;
-    if (alive && (mode == kCmScratch || mode == kCmContinue)) {
-        CgStart start{};
-        if (mode == kCmContinue) {
-            // r_k into the buffer iteration k reads, p_{k-1} likewise (k is odd)
-            cm_pass2_any(g, plan.k, wfirst, warps, plan.qr, a.r[1]);
-            cm_pass2_any(g, plan.k - 1, wfirst, warps, plan.qp, a.p[0]);
-            start.k = plan.k;
-            start.alpha = plan.alpha;
-            start.alpha_prev = plan.alpha_prev;
-            start.beta = plan.beta;
-            start.absNew = plan.absNew;
-            start.pAp = plan.pAp;
-            start.bb = plan.bb;
-            start.threshold = plan.threshold;
-        }
-        if (a.start) {  // the CG kernel launched next takes over
-            report = false;
-            if (blockIdx.x == 0 && tid == 0) *a.start = start;
-        } else {
-            __syncthreads();  // the rings change their layout
-            if (mode == kCmScratch || barrier()) {
-                const int strips = (g.nx + CG_W - 1) / CG_W;
-                const int segs = max(1, warps / strips);
-                const int seg_h = max(4, (g.ny + segs - 1) / segs);
-                // (partials of its own: other blocks may still read the moments')
-                cg_iterate<CM_NT, false, true>(a, strips, seg_h, strips * ((g.ny + seg_h - 1) / seg_h), s,
-                                  cm_warp_smem(), a.partials + (size_t)CM_NMU * G, &red[0][0],
-                                  scal, barrier, start, res);
-            }
-            report = alive;
-        }
-    } else if (alive) {
-        res.products = (mode == kCmDone || mode == kCmCapped) ? plan.k : 0;
-        res.bb = plan.bb;
-        res.rr = plan.rr;
-        res.breakdown = mode == kCmBreakdown;
-        res.converged = mode == kCmDone || mode == kCmZero;
-        if (mode == kCmZero || mode == kCmBreakdown) {
-            const size_t n = (size_t)g.nx * g.ny;
-            for (size_t e = (size_t)blockIdx.x * CM_NT + tid; e < n; e += (size_t)G * CM_NT) a.x[e] = 0.0;
-        }
-    }
-    if (blockIdx.x == 0 && tid == 0) {
-        if (report) cg_report(a, res);
-        // solved, or given up: nothing is left for the CG kernel
-        if (a.start && (report || !alive)) a.start->k = -1;
-    }
-}
-
 }  // namespace mhd

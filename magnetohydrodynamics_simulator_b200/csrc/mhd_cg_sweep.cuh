@@ -535,39 +535,4 @@ __device__ __forceinline__ void cg_report(const CgSweepArgs& a, const CgResult& 
     else if (!r.converged) atomicOr(&a.st->flags, (unsigned)kStatusCgNotConverged);
 }
 
-// START: behind k_solve, which says in a.start what is left to do.
-template <bool START>
-__global__ void __launch_bounds__(CGS_NT, MHD_CG_MIN_BLOCKS)
-k_cg_sweep(const __grid_constant__ CgSweepArgs a) {
-    __shared__ double red[CGS_NT / 32 * 4];
-    __shared__ double scal[8];
-    __shared__ int sflag;
-#if defined(__CUDA_ARCH__)
-    extern __shared__ __align__(16) double cg_ring_mem[];
-#else
-    // host compilation of the kernel sources (single-block logic tests): one shared copy
-    static double cg_ring_mem[(CGS_NT / 32) * CG_RING * CG_SLOT];
-#endif
-    CgStart start{};
-    if constexpr (START) {
-        start = *a.start;
-        if (start.k < 0) return;
-    }
-    double* const ring = cg_ring_mem + (size_t)(threadIdx.x >> 5) * CG_RING * CG_SLOT;
-    const int tid = threadIdx.x;
-    CgScal s = cg_scalars(a);
-    unsigned long long target = barrier_base(a.sync);
-    const unsigned long long deadline =
-        global_timer_ns() + (unsigned long long)(a.timeout_s * 1e9);
-    auto barrier = [&]() -> bool {
-        if (grid_barrier(a.sync, target, deadline, &sflag)) return true;
-        // (any block: one that gives up leaves its part undone)
-        if (tid == 0) atomicOr(&a.st->flags, (unsigned)kStatusTimeout);
-        return false;
-    };
-    CgResult res{};
-    if (cg_iterate<CGS_NT, true, START>(a, a.strips_x, a.seg_h, a.nwarps, s, ring, a.partials, red, scal, barrier, start, res) && blockIdx.x == 0 && tid == 0)
-        cg_report(a, res);
-}
-
 }  // namespace mhd
