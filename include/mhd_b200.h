@@ -184,8 +184,8 @@ mhd_status mhd_kernel_times(mhd_context* ctx, double out_ms[5], long long* steps
 /* The stream the context enqueues on (a cudaStream_t). */
 void* mhd_stream(mhd_context* ctx);
 
-/* Number of kernel launches one mhd_step with a device-chosen dt enqueues (for launch accounting); a solve whose dt
- * the caller gives is one launch less on grids that are too large for one thread-block cluster. */
+/* Number of kernel launches one mhd_step with a device-chosen dt enqueues (for launch accounting); with a dt that the
+ * caller gives a solve can be one launch less on grids that are too large for one thread-block cluster. */
 int mhd_launches_per_step(mhd_context* ctx);
 
 /* Snapshots in the reference's file format: the bytes write_data_to_binary_file

@@ -21,8 +21,9 @@
 // running error bound (the sums' relative error is far below kCmNoise), and only norms well above
 // it are used. If the residual has not passed the threshold at the last usable k, the ordinary
 // iterations go on from there: r, p and x of an earlier iterate are evaluated from their polynomials
-// (three more passes) and the sweeps of mhd_cg_sweep.cuh go on, in this kernel or in the CG kernel launched
-// behind it. With no usable norm, or beyond kCmMaxT, they start from the right-hand side.
+// (three more passes) and the sweeps of mhd_cg_sweep.cuh go on, in k_solve or in the k_cg_sweep launched
+// behind it. With no usable norm, beyond kCmMaxT, or in front of a k_cg_band, which takes up no iterate (it
+// gains nothing by the passes then: beyond kCmSureT), they start from the right-hand side.
 //
 // Bound by instruction issue at two warps a scheduler (FP64 pipe 40%, DRAM 30%), not by DRAM. Measured on
 // B200, one solve: 4096^2, eta 1e-4 (6 products) 792 -> 308 us; 2048^2, eta 1e-3 (9 products) 360 -> 172 us;
@@ -56,12 +57,16 @@ static_assert(CG_RING * CG_SLOT <= CM_WARP, "the sweeps' rings fit the passes' s
 constexpr double kCmNoise = 5.7e-14;  // relative error allowed to the moment sums (256 eps)
 constexpr double kCmTrust = 8.0;      // a norm counts when it exceeds its error bound this many times
 constexpr double kCmMaxT = 0.06;      // largest t = 2 (cx + cy) of the moment form
+constexpr double kCmSureT = 0.033;    // beyond it CM_MAXM levels may not suffice (cm_levels)
 
 // Levels of pass 1. The a-priori CG bound, 2 sqrt(kappa) zeta^k with zeta = (sqrt(kappa) - 1) / (sqrt(kappa)
-// + 1) and kappa = 1 + 2 t, reaches machine precision by k = 5 up to t = 1.2e-3 and by k = 7 up to t = 0.0105;
-// flows need one product less (7 at t = 0.0155, 9 at 0.053). Where the levels do not suffice the ordinary
-// iterations finish.
-__device__ __forceinline__ int cm_levels(double t) { return t < 1.2e-3 ? 5 : (t < 0.0155 ? 7 : CM_MAXM); }
+// + 1) and kappa = 1 + 2 t, reaches machine precision by k = 5 up to t = 1.2e-3, by k = 7 up to t = 0.0105 and by
+// k = 9 up to 0.034; flows need one product less (7 at t = 0.0155, 9 at 0.053), noise does not. Where the levels do
+// not suffice the ordinary iterations finish. (9 levels from 0.0105 on: a CFL step of a flow at 512^2 takes 159 us for
+// 144, one of a noisy field 168 for 246.)
+__host__ __device__ inline int cm_levels(double t) { return t < 1.2e-3 ? 5 : (t < 0.0155 ? 7 : CM_MAXM); }
+// Whether they suffice for any right-hand side.
+__host__ __device__ inline bool cm_sure(double t) { return t < 0.0105 || (t >= 0.0155 && t <= kCmSureT); }
 
 struct CmSpan {
     int strips, seg_h, n;  // column strips, rows per segment, segments in all

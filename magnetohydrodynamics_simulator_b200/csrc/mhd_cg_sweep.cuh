@@ -50,7 +50,8 @@ struct CgSweepArgs {
     double* p[2];
     double* partials;  // [2][gridDim.x][4]
     CgSync* sync;
-    struct CgStart* start;  // where k_cg_sweep, launched behind k_solve, enters (null: it is not)
+    struct CgStart* start;  // where the CG kernel launched behind k_solve enters (null: there is none)
+    bool from_rhs;          // ... and can only start from the right-hand side
     DeviceStatus* st;
     long long* prods_out;
     int solve_index;

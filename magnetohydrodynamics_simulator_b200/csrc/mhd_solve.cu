@@ -70,7 +70,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     CgScal s = cg_scalars(a);
     const double t = 2 * (s.cx + s.cy);
-    const bool in_range = t >= 1e-30 && t <= kCmMaxT;
+    const bool in_range = t >= 1e-30 && t <= (a.from_rhs ? kCmSureT : kCmMaxT);
     if (a.start && !in_range) {  // the CG kernel launched next does all of it
         if (blockIdx.x == 0 && tid == 0) a.start->k = 0;
         return;
@@ -119,6 +119,7 @@ k_solve(const __grid_constant__ CgSweepArgs a) {
             if (wid == 0) cm_plan(mu[lane], M, t, s.diag, scale, a.tol, a.max_iters, &plan);
             __syncthreads();
             mode = plan.mode;
+            if (mode == kCmContinue && a.from_rhs) mode = kCmScratch;
             if (mode == kCmDone || mode == kCmCapped || mode == kCmContinue)
                 cm_pass2_any(g, plan.k - 1, wfirst, warps, plan.q, a.x);
         }
@@ -278,9 +279,10 @@ mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool f
     a.strips_x = g.strips_x;
     a.seg_h = g.seg_h;
     a.nwarps = g.nwarps;
-    const bool moments = t <= mhd::kCmMaxT && !(field && (long long)a.D.nx * a.D.ny < (1 << 21));
-    const bool sweep = t < 0.0 || !moments;
-    a.start = (t < 0.0 && sweep) ? &dev->start : nullptr;
+    const bool moments = t <= (g.band ? mhd::kCmSureT : mhd::kCmMaxT) && !(field && (long long)a.D.nx * a.D.ny < (1 << 21));
+    const bool sweep = t < 0.0 || !moments || !mhd::cm_sure(t);
+    a.start = moments && sweep ? &dev->start : nullptr;
+    a.from_rhs = a.start && g.band;
     if (moments) {
         a.sync = &dev->sync[0];
         cfg.gridDim = dim3(g.mgrid);

@@ -38,11 +38,15 @@ inline double solve_t(double alpha, double dx, double dy) {
 }
 
 // Launch the solve of `a` (its geometry, sync and start are set here). t: solve_t where the host knows
-// alpha, else negative (the step's dt is chosen on the device). Up to kCmMaxT k_solve alone (two passes
-// over the face planes), beyond it CG alone: k_cg_band where the chip's shared memory holds the grid, else
-// k_cg_sweep (one sweep per product). Where the host does not know, k_solve comes first and CG behind it
-// finds the solve done, or does it: an idle kernel costs 1 us. (k_cg_band starts from the right-hand side;
-// k_cg_sweep also takes up an iteration that k_solve left.)
+// alpha, else negative (the step's dt is chosen on the device).
+// Up to kCmSureT k_solve (two passes over the face planes). Beyond it the levels may not suffice, and the passes are then
+// lost: grids that the chip's shared memory holds take k_cg_band (steps of fixed dt at t = 0.06, 10 products a solve, with
+// the two passes first and with k_cg_band alone: 300^2 249 and 156 us, 512^2 307 and 197, 1000^2 619 and 363; with 9
+// products, which the passes settle, 177 and 143, 168 and 179, 343 and 330), larger ones k_solve up to kCmMaxT and
+// k_cg_sweep (one sweep per product) after that.
+// A CG kernel behind k_solve finds the solve done, or does it: where the host does not know t, and where the levels are
+// not sure to suffice. An idle kernel costs 4 us; without it k_solve goes on with sweeps of its own, which are slower
+// (t = 0.06, 10 products: a step at 1448^2 900 us, 780 with k_cg_sweep behind).
 // Grids that fit one cluster take k_cg_cluster, whatever the matrix.
 // field: the right-hand side is a caller's field, not an evolved one. Smooth fields take two to four products,
 // and below 1448^2 as many are shorter than the two passes, whose length does not depend on them
