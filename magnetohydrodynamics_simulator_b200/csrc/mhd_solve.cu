@@ -254,6 +254,21 @@ SolveGeom solve_geometry(int nx, int ny, int num_sms) {
     return g;
 }
 
+// Cells from which on a caller's field takes the two passes. Their length does not depend on the field; smooth fields of
+// few modes take two products up to t = 8e-3 or so and three or four beyond, and the sweeps are then shorter up to the
+// grids below (k_cg_sweep against k_solve, us a call):
+//   t = 1e-3, 2 products   1800^2 130, 141   2048^2 155, 166   2200^2 176, 172   2700^2 239, 215
+//   t = 2e-3, 2 products   2048^2 156, 177   2400^2 205, 217   2700^2 252, 256
+//   t = 1e-2, 3 products   1500^2 141, 131   2048^2 219, 179
+//   t = 0.03, 3 products   1500^2 142, 154   1600^2 156, 160   1800^2 188, 178   2048^2 226, 203
+//   t = 0.05, 4 products   1600^2 157, 158   1800^2 185, 181   2048^2 224, 206
+// (noise, 4 to 9 products, gains from the two passes on any of these: 1.2 to 2 times.)
+static long long field_line(double t) {
+    if (t < 1.2e-3) return 4800000;
+    if (t < 8e-3) return 7000000;
+    return t < 0.0155 ? 1 << 21 : 2900000;
+}
+
 mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool field, SolveSync* dev,
                         cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
@@ -279,7 +294,8 @@ mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool f
     a.strips_x = g.strips_x;
     a.seg_h = g.seg_h;
     a.nwarps = g.nwarps;
-    const bool moments = t <= (g.band ? mhd::kCmSureT : mhd::kCmMaxT) && !(field && (long long)a.D.nx * a.D.ny < (1 << 21));
+    const bool moments = t <= (g.band ? mhd::kCmSureT : mhd::kCmMaxT) &&
+                         !(field && (long long)a.D.nx * a.D.ny < field_line(t));
     const bool sweep = t < 0.0 || !moments || !mhd::cm_sure(t);
     a.start = moments && sweep ? &dev->start : nullptr;
     a.from_rhs = a.start && g.band;

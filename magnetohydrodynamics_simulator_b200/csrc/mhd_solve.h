@@ -48,9 +48,8 @@ inline double solve_t(double alpha, double dx, double dy) {
 // not sure to suffice. An idle kernel costs 4 us; without it k_solve goes on with sweeps of its own, which are slower
 // (t = 0.06, 10 products: a step at 1448^2 900 us, 780 with k_cg_sweep behind).
 // Grids that fit one cluster take k_cg_cluster, whatever the matrix.
-// field: the right-hand side is a caller's field, not an evolved one. Smooth fields take two to four products,
-// and below 1448^2 as many are shorter than the two passes, whose length does not depend on them
-// (1024^2 with k_cg_sweep: 3 products 66 against 76 us; 2048^2: 198 against 154); in a step there are five or more.
+// field: the right-hand side is a caller's field, not an evolved one, which in a step takes five products or more: below
+// field_line(t) cells it takes CG alone.
 mhd_status launch_solve(mhd::CgSweepArgs a, const SolveGeom& g, double t, bool field, SolveSync* dev,
                         cudaStream_t stream);
 
