@@ -545,11 +545,19 @@ mhd_status mhd_adj_rate_vjp(mhd_adjoint* a, const double* const u[6], const doub
     if (!u || !w || !out) return MHD_ERR_INVALID_ARGUMENT;
     for (int k = 0; k < 6; ++k)
         if (!u[k] || !w[k] || !out[k]) return MHD_ERR_INVALID_ARGUMENT;
-    // the sweep reads U and w around the cells it writes: through scratch, so that out may be u or w
+    // the sweep reads u and w around the cells it writes: where out lies over one of them, by way of scratch
+    bool over = false;
+    for (int k = 0; k < 6; ++k)
+        for (int q = 0; q < 6; ++q)
+            over |= mhd_host::overlap(out[k], u[q], a->n * sizeof(double)) ||
+                    mhd_host::overlap(out[k], w[q], a->n * sizeof(double));
+    double* const* const to = over ? a->s.lamT : out;
     const double* const zero[6] = {};
-    if ((s = rate_vjp(a, u, w, 1.0, zero, a->s.lamT)) != MHD_OK) return s;
-    const double* const r[6] = {a->s.lamT[0], a->s.lamT[1], a->s.lamT[2], a->s.lamT[3], a->s.lamT[4], a->s.lamT[5]};
-    if ((s = copy_planes(a, out, r)) != MHD_OK) return s;
+    if ((s = rate_vjp(a, u, w, 1.0, zero, to)) != MHD_OK) return s;
+    if (over) {
+        const double* const r[6] = {to[0], to[1], to[2], to[3], to[4], to[5]};
+        if ((s = copy_planes(a, out, r)) != MHD_OK) return s;
+    }
     MHD_TRY(cudaStreamSynchronize(a->stream));
     return MHD_OK;
 }

@@ -7,6 +7,7 @@
 #include <nvtx3/nvToolsExt.h>
 #endif
 
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 
@@ -26,6 +27,12 @@ inline mhd_status cuda_status(cudaError_t e) {
 inline int env_int(const char* name, int def) {
     const char* v = getenv(name);
     return v ? atoi(v) : def;
+}
+
+// Whether two planes of `bytes` share any.
+inline bool overlap(const void* p, const void* q, size_t bytes) {
+    const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
+    return a < b + bytes && b < a + bytes;
 }
 
 // An NVTX range over one entry point's host work (what it enqueues shows under it in a timeline

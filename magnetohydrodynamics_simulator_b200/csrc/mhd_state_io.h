@@ -87,11 +87,6 @@ inline bool plain_device_range(const void* p, size_t bytes, int device) {
            a - base <= size && bytes <= size - (a - base);
 }
 
-inline bool overlap(const void* p, const void* q, size_t bytes) {
-    const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
-    return a < b + bytes && b < a + bytes;
-}
-
 // The six planes f (null: skipped) for a kernel that moves them to or from the planes s: plain memory, apart from
 // s and, when written, from one another.
 inline bool plain_state(const double* const* f, const double* const* s, size_t bytes, int device, bool written) {
