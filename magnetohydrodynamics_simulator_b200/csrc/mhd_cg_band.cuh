@@ -27,24 +27,33 @@ constexpr int CB_SMEM_DOUBLES = 28672;   // 224 KB
 // off the chip (200 x 200, three fixed steps, three contexts on three streams: 499 us with two-row bands, 219 with
 // 1600 cells, 251 with 3200; one alone 649, 627 and 737).
 constexpr int CB_MIN_CELLS = 1600;
-// Up to this many cells a band takes half the SMs: a solve is 10-14% longer, but two run side by side (512^2 at
-// eta 10, two fixed steps: 3.43 ms a context on 128 SMs, 1.96 on 73; one alone 3.54 and 3.89).
-constexpr int CB_HALF_CELLS = 3600;
 // Doubles of dynamic shared memory of a block whose band has at most R rows.
 __host__ __device__ constexpr long long cb_smem_doubles(long long nx, long long R) { return nx * (3 * R + 4); }
 
 // Bands of an nx x ny grid on num_sms SMs; 0: does not fit. Every band has two rows or more (their edge rows share
 // the planes a.r with room for two a band).
+// Half of the SMs where their shared memory holds the grid (up to some 680^2): a solve is then up to 15% longer, but two
+// run side by side. A step of fixed dt at eta 10 (257 to 423 products), one context alone, and each of three on streams
+// of their own, in us, with bands for all SMs and for half of them:
+//            400^2       450^2       512^2       520^2       560^2       600^2       640^2       660^2
+//   alone  1320 1407   1590 1573   1729 1887   2037 2262   2265 2423   2695 2820   2794 2937   3107 3149
+//   three  1256  687   1565  769   1684  964   2002 1112   2232 1193   2649 1384   2746 1471   3058 1625
+//          682x888     1000x592    1024x592    1024x444    512x888     400x1100    300x1400
+//   alone  3998 3973   3660 4179   3725 4274   3454 3840   3036 3277   3717 3896   4262 4690
+//   three  4015 2041   3669 2130   3738 2172   3459 1963   3055 1663   3697 1969   4270 2368
+// (up to 350^2 CB_MIN_CELLS makes the bands, the same for both.)
 inline int cb_bands(int nx, int ny, int num_sms) {
     if (ny < 2 || nx < 2) return 0;
-    const int half = (2 * ny + num_sms - 1) / num_sms;
-    const int R = std::max({2, (long long)nx * half <= CB_HALF_CELLS ? half : (ny + num_sms - 1) / num_sms,
-                            (CB_MIN_CELLS + nx - 1) / nx});
-    const int bands = std::max(1, std::min(ny / R, num_sms));
-    const long long Rmax = (ny + bands - 1) / bands;
-    return cb_smem_doubles(nx, Rmax) <= CB_SMEM_DOUBLES &&
-                   (long long)nx * ((Rmax + CB_V - 1) / CB_V) <= (long long)CB_ITEMS * CB_NT
-               ? bands : 0;
+    auto fit = [&](int sms) {
+        const int R = std::max({2, (ny + sms - 1) / sms, (CB_MIN_CELLS + nx - 1) / nx});
+        const int bands = std::max(1, std::min(ny / R, num_sms));
+        const long long Rmax = (ny + bands - 1) / bands;
+        return cb_smem_doubles(nx, Rmax) <= CB_SMEM_DOUBLES &&
+                       (long long)nx * ((Rmax + CB_V - 1) / CB_V) <= (long long)CB_ITEMS * CB_NT
+                   ? bands : 0;
+    };
+    const int half = fit(std::max(1, num_sms / 2));
+    return half ? half : fit(num_sms);
 }
 
 struct CbShared {

@@ -94,3 +94,19 @@ def test_step_on_either_side_of_the_two_pass_forms_range(m, t, kind, few):
     assert (max(a.last_cg_products()) <= 9) == few
     for u, v in zip(a.get_state(), b.get_state()):
         assert np.array_equal(u, v)
+
+
+@pytest.mark.parametrize("shape", [(682, 888), (683, 888), (512, 512), (520, 521), (1365, 290), (1024, 592), (1025, 592)])
+def test_rate_on_half_the_chip_and_on_all_of_it(m, shape):
+    """The largest grids whose bands fit half of the SMs, and the next ones (four and two runs a thread)."""
+    nx, ny = shape
+    dx, dy, eta = 2 * np.pi / nx, 1.3 * 2 * np.pi / ny, 0.7
+    alpha = 0.3 / (2 * (1 / dx**2 + 1 / dy**2))
+    bx, by = _faces(nx, ny, dx, dy, "noise", seed=nx * 31 + ny)
+    gx, gy, prods, status = _rate(m, nx, ny, dx, dy, eta, alpha, bx, by)
+    x, k = _cg(bx, by, dx, dy, eta, alpha)
+    assert status == 0
+    assert abs(prods - k) <= 1, (prods, k)
+    bound = 64 * EPS * np.abs(x).max() / min(dx, dy)
+    assert np.abs(gx + (np.roll(x, -1, 0) - x) / dy).max() <= bound
+    assert np.abs(gy - (np.roll(x, -1, 1) - x) / dx).max() <= bound
