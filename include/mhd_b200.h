@@ -213,7 +213,7 @@ mhd_status mhd_snapshot_pack(mhd_context* ctx, int ng, int snapshot_rate, double
  * `count` independent periodic simulations, each with its own mhd_params (size, spacing, eta,
  * courant, safety, ct_mode, solver tolerance), advanced together. Each step is one launch per
  * stage for the whole batch (coefficients, stage 1, implicit solve, stage 2, implicit solve,
- * finalize; the solves take one launch per 64 instances). Every instance gets exactly the step
+ * finalize; the solves take up to three launches per 64 instances). Every instance gets exactly the step
  * it would get from its own mhd_context: its own CFL dt, its own matrix coefficient, its own CG
  * convergence. States are dense nx*ny planes in the order rho, mx, my, E, bxf, byf. */
 typedef struct mhd_batch mhd_batch;

@@ -815,8 +815,9 @@ mhd_status mhd_batch_get_tuning(mhd_batch* b, mhd_batch_tuning* t) {
 
 // Autotuner: one CFL step of the current states per candidate, timed per kernel with events;
 // the explicit-stage (row height, tail height) and the solver's (row height, dealing order) are chosen
-// independently (they set disjoint kernels' decompositions). States, device statuses, step
-// coefficients and the descriptor parity are restored after every trial.
+// independently (they set disjoint kernels' decompositions). The solver's only sets k_cg_batch's: it stays as it is
+// where the other forms settle every instance, so that a later solve's summation order does not hang on the noise of
+// equal trials. States, device statuses, step coefficients and the descriptor parity are restored after every trial.
 mhd_status mhd_batch_autotune(mhd_batch* b, mhd_batch_tuning* out) {
     mhd_status s = check_batch(b);
     if (s != MHD_OK) return s;
@@ -861,6 +862,8 @@ mhd_status mhd_batch_autotune(mhd_batch* b, mhd_batch_tuning* out) {
                                 b->count * sizeof(StepCoeffs), cudaMemcpyDeviceToDevice, b->stream));
         MHD_TRY(cudaMemcpyAsync(save ? status_bk : b->status, save ? b->status : status_bk,
                                 b->count * sizeof(DeviceStatus), cudaMemcpyDeviceToDevice, b->stream));
+        // (a trial whose solve ran out of time: its status goes, so its barrier does)
+        if (!save) MHD_TRY(cudaMemsetAsync(b->solve_syncs, 0, (size_t)b->nchunks * sizeof(CgSync), b->stream));
         b->parity = parity0;
         return MHD_OK;
     };
@@ -874,23 +877,30 @@ mhd_status mhd_batch_autotune(mhd_batch* b, mhd_batch_tuning* out) {
     double best_stage = 1e300, best_cg = 1e300;
     int best_stage_rows = before.stage_rows, best_tail = before.stage_tail_rows;
     int best_cg_rows = before.cg_rows, best_order = before.cg_order;
-    // trial -1 warms the kernels up; the others cover every solver candidate and every
-    // explicit-stage candidate
-    const int ntrials = std::max(nst, ncg);
+    // trial -1 warms the kernels up; the others cover every explicit-stage candidate and, where it has work, every
+    // solver candidate
+    int ntrials = nst;
+    bool solver = false;  // the step's second solve (the last to set todo) leaves an instance to k_cg_batch
     for (int trial = -1; trial < ntrials; ++trial) {
         mhd_batch_tuning t{};
         const int tk = std::max(trial, 0);
         t.stage_rows = stage_cand[tk % nst].first;
         t.stage_tail_rows = stage_cand[tk % nst].second;
-        t.cg_rows = kCgCand[tk % ncg][0];
-        t.cg_order = kCgCand[tk % ncg][1];
+        t.cg_rows = solver ? kCgCand[tk % ncg][0] : before.cg_rows;
+        t.cg_order = solver ? kCgCand[tk % ncg][1] : before.cg_order;
         if ((s = apply_tuning(b, t)) != MHD_OK) return s;
         if ((s = enqueue_step(b, nullptr, 0.0, 1, 0.0, false, ev)) != MHD_OK) return s;
         MHD_TRY(cudaStreamSynchronize(b->stream));
         float ms[5];
         for (int k = 0; k < 5; ++k) MHD_TRY(cudaEventElapsedTime(&ms[k], ev[k], ev[k + 1]));
         if ((s = planes_copy(false)) != MHD_OK) return s;
-        if (trial < 0) continue;
+        if (trial < 0) {
+            std::vector<int> todo(b->count);
+            MHD_TRY(cudaMemcpy(todo.data(), b->todo, b->count * sizeof(int), cudaMemcpyDeviceToHost));
+            solver = std::any_of(todo.begin(), todo.end(), [](int v) { return v != 0; });
+            if (solver) ntrials = std::max(nst, ncg);
+            continue;
+        }
         const double stage_ms = (double)ms[0] + ms[2] + ms[4];
         const double cg_ms = (double)ms[1] + ms[3];
         if (stage_ms < best_stage) {
