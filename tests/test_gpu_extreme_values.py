@@ -207,3 +207,31 @@ def test_rate_vjp_in_far_units(m, rho, v, v0):
         err = float((out[k].cpu() - want[k]).abs().max() / want[k].abs().max())
         assert err <= 1e-9, (k, err)
     adj.close()
+
+
+# grids whose solves take the two passes, the chip's shared memory (t > 0.06) and, larger, the sweeps
+@pytest.mark.parametrize("nx,ny,eta", [(300, 290, 1e-4), (300, 290, 0.5), (1300, 1000, 1e-4), (1300, 1000, 0.5)])
+@pytest.mark.parametrize("dt", [0.0, 1e-4])
+def test_solve_of_a_bad_field_is_reported(m, nx, ny, eta, dt):
+    """A NaN in the field breaks every form of the solve down: the status says so, and the next state steps on."""
+    dx, dy = 2 * np.pi / nx, 2 * np.pi / ny
+    ic = m.problems.orszag_tang(nx, ny, dx, dy)
+    bad = [f.copy() for f in ic]
+    bad[4][ny // 3, nx // 2] = np.nan
+    ctx = m.Context(nx, ny, dx, dy, eta)
+    batch = m.Batch([{"nx": n, "ny": k, "dx": dx, "dy": dy, "eta": eta} for n, k in ((nx, ny), (nx, ny))])
+    ctx.set_state(bad)
+    batch.set_state(0, bad)
+    batch.set_state(1, ic)
+    ctx.step(dt)
+    assert ctx.synchronize_status() == 3  # MHD_ERR_NONFINITE
+    batch.step([dt, dt] if dt else None)
+    worst, each = batch.synchronize_status()
+    assert worst == 3 and list(each) == [3, 0]
+    ctx.set_state(ic)
+    ctx.step(dt)
+    assert ctx.synchronize_status() == 0
+    for g, w in zip(batch.get_state(1), ctx.get_state()):
+        assert np.abs(g - w).max() <= 1e-12 * max(np.abs(w).max(), 1.0)
+    ctx.close()
+    batch.close()
