@@ -287,7 +287,7 @@ int mhd_device_available(void) {
         return 0;
     }
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k_finalize) != cudaSuccess) {
+    if (cudaFuncGetAttributes(&fa, k_driver_reset) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }

@@ -1,6 +1,6 @@
 // Shared device code of the ARS(2,2,2) IMEX step (reference: solvers.hpp:491-613 of
 // RikibabManos/Magnetohydrodynamics_Simulator), for sm_100a, FP64: parameter blocks, helpers,
-// the bounded grid barrier, the step-coefficient / driver kernel, the finalize kernel and the
+// the bounded grid barrier, the step-coefficient / driver kernel, the CFL scan and the
 // diagnostics. The explicit stages live in mhd_sweep.cuh, the finalize in mhd_finalize_sweep.cuh, the implicit
 // solve in mhd_cg_cluster.cuh (small grids), mhd_cg_moments.cuh (small t), mhd_cg_band.cuh and mhd_cg_sweep.cuh
 // (the rest); mhd_solve.h chooses.
@@ -178,7 +178,7 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* red) {
 
 // Grid barrier of a cooperatively launched kernel, with a wall-clock limit: returns false when the
 // caller must stop (time ran out here or in another block); the caller then returns without
-// touching shared state again. The counter is zeroed before each launch.
+// touching shared state again. The counter is zeroed before a launch, or target starts at barrier_base.
 __device__ __forceinline__ bool grid_barrier(CgSync* sync, unsigned long long& target,
                                              unsigned long long deadline, int* sflag) {
     __syncthreads();
@@ -323,110 +323,6 @@ static __global__ void k_step_coeffs(StepCoeffs* C, DeviceStatus* st, double dt,
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     step_coeffs_one(C, st, dt, alpha, alpha_mode, eta, hmin, courant, safety, g, d, t_end, dts_out);
     st->smax_bits = 0ULL;
-}
-
-// ------------------------------------------------------------------------------------------
-// Finalize: B2 = U2*_B + dt*g*rate(E2); g3 = explicit resistive rate of B2;
-// B^{n+1} = U2*_B + dt*g*g3 (solvers.hpp:571-608); density floor of the new state in place
-// (solvers.hpp:610-611); max CFL signal speed (diagnostics.hpp:60-78); non-finite check.
-
-constexpr int FN_TX = 32, FN_TY = 16, FN_NT = 256;
-constexpr int FN_XW = FN_TX + 4, FN_XH = FN_TY + 4;   // E2 over [i0-1, i0+TX+2] x [j0-1, j0+TY+2]
-constexpr int FN_BXW = FN_TX + 2, FN_BXH = FN_TY + 3;  // bxf over [i0, i0+TX+1] x [j0-1, j0+TY+1]
-constexpr int FN_BYW = FN_TX + 3, FN_BYH = FN_TY + 2;  // byf over [i0-1, i0+TX+1] x [j0, j0+TY+1]
-constexpr int FN_EW = FN_TX + 2, FN_EH = FN_TY + 2;    // E3 corners [i0, i0+TX+1] x [j0, j0+TY+1]
-constexpr int FN_NW = FN_TX + 1, FN_NH = FN_TY + 1;    // B^{n+1} on cells [i0, i0+TX] x [j0, j0+TY]
-
-struct FinalSmem {
-    double x[FN_XW * FN_XH];
-    double bx0[FN_BXW * FN_BXH], by0[FN_BYW * FN_BYH];  // U2*_B
-    double bx2[FN_BXW * FN_BXH], by2[FN_BYW * FN_BYH];  // B2
-    double e3[FN_EW * FN_EH];
-    double bxn[FN_NW * FN_NH], byn[FN_NW * FN_NH];
-    double red[32];
-};
-
-static __global__ void __launch_bounds__(FN_NT)
-k_finalize(Domain D, const StepCoeffs* __restrict__ C, Planes acc, const double* __restrict__ xsolve,
-           double* __restrict__ bx_out, double* __restrict__ by_out, DeviceStatus* st, int tiles_x) {
-    __shared__ FinalSmem s;
-    const int tid = threadIdx.x;
-    const int i0 = (blockIdx.x % tiles_x) * FN_TX;
-    const int j0 = (blockIdx.x / tiles_x) * FN_TY;
-    const int nx = D.nx, ny = D.ny;
-    for (int k = tid; k < FN_XW * FN_XH; k += FN_NT) {
-        const int jj = k / FN_XW, ii = k - jj * FN_XW;
-        s.x[k] = xsolve[(size_t)wrap(j0 - 1 + jj, ny) * nx + wrap(i0 - 1 + ii, nx)];
-    }
-    for (int k = tid; k < FN_BXW * FN_BXH; k += FN_NT) {
-        const int jj = k / FN_BXW, ii = k - jj * FN_BXW;
-        s.bx0[k] = acc.f[4][(size_t)wrap(j0 - 1 + jj, ny) * nx + wrap(i0 + ii, nx)];
-    }
-    for (int k = tid; k < FN_BYW * FN_BYH; k += FN_NT) {
-        const int jj = k / FN_BYW, ii = k - jj * FN_BYW;
-        s.by0[k] = acc.f[5][(size_t)wrap(j0 + jj, ny) * nx + wrap(i0 - 1 + ii, nx)];
-    }
-    __syncthreads();
-    const double cg = C->c_g;
-    // B2 (solvers.hpp:573-574); x index of corner (i,j) = (j - j0 + 1) * XW + (i - i0 + 1)
-    for (int k = tid; k < FN_BXW * FN_BXH; k += FN_NT) {
-        const int jj = k / FN_BXW, ii = k - jj * FN_BXW;  // face (i0+ii, j0-1+jj)
-        const int xc = jj * FN_XW + ii + 1;
-        const double rate = -(s.x[xc + FN_XW] - s.x[xc]) / D.dy;
-        s.bx2[k] = s.bx0[k] + rate * cg;
-    }
-    for (int k = tid; k < FN_BYW * FN_BYH; k += FN_NT) {
-        const int jj = k / FN_BYW, ii = k - jj * FN_BYW;  // face (i0-1+ii, j0+jj)
-        const int xc = (jj + 1) * FN_XW + ii;
-        const double rate = (s.x[xc + 1] - s.x[xc]) / D.dx;
-        s.by2[k] = s.by0[k] + rate * cg;
-    }
-    __syncthreads();
-    // E3 = eta J_z(B2) at corners (i0+ei, j0+ej) (solvers.hpp:450-461)
-    for (int k = tid; k < FN_EW * FN_EH; k += FN_NT) {
-        const int ej = k / FN_EW, ei = k - ej * FN_EW;
-        const int cyy = ej * FN_BYW + ei + 1;        // byf(i, j): col i-(i0-1), row j-j0
-        const int cxx = (ej + 1) * FN_BXW + ei;      // bxf(i, j): col i-i0, row j-(j0-1)
-        const double dBy_dx = (s.by2[cyy] - s.by2[cyy - 1]) / D.dx;
-        const double dBx_dy = (s.bx2[cxx] - s.bx2[cxx - FN_BXW]) / D.dy;
-        s.e3[k] = D.eta * (dBy_dx - dBx_dy);
-    }
-    __syncthreads();
-    // B^{n+1} = U2*_B + dt*g * g3 on cells [i0, i0+TX] x [j0, j0+TY] (solvers.hpp:607-608)
-    for (int k = tid; k < FN_NW * FN_NH; k += FN_NT) {
-        const int nj = k / FN_NW, ni = k - nj * FN_NW;
-        const int e = nj * FN_EW + ni;
-        const double g3x = -(s.e3[e + FN_EW] - s.e3[e]) / D.dy;
-        const double g3y = (s.e3[e + 1] - s.e3[e]) / D.dx;
-        s.bxn[k] = s.bx0[(nj + 1) * FN_BXW + ni] + g3x * cg;
-        s.byn[k] = s.by0[nj * FN_BYW + ni + 1] + g3y * cg;
-    }
-    __syncthreads();
-    double vmax = 0.0;
-    bool bad = false;
-    for (int k = tid; k < FN_TX * FN_TY; k += FN_NT) {
-        const int tj = k / FN_TX, ti = k - tj * FN_TX;
-        const int i = i0 + ti, j = j0 + tj;
-        if (i >= nx || j >= ny) continue;
-        const size_t g = (size_t)j * nx + i;
-        const int n = tj * FN_NW + ti;
-        const double bx = s.bxn[n], by = s.byn[n];
-        bx_out[g] = bx;
-        by_out[g] = by;
-        // primitives of the new state (Grid.hpp:100-136), then the CFL speed of the cell
-        double rho = acc.f[0][g];
-        const double mx = acc.f[1][g], my = acc.f[2][g], E = acc.f[3][g];
-        if (rho < kRhoFloor) acc.f[0][g] = kRhoFloor;
-        const double bxc = (bx + s.bxn[n + 1]) / 2.0;
-        const double byc = (by + s.byn[n + FN_NW]) / 2.0;
-        const double sp = cell_cfl_speed(rho, mx, my, E, bxc, byc);
-        if (sp > vmax) vmax = sp;
-        bad |= !(isfinite(rho) && isfinite(mx) && isfinite(my) && isfinite(E) && isfinite(bx) &&
-                 isfinite(by));
-    }
-    vmax = block_max<FN_NT>(vmax, s.red);
-    if (__syncthreads_or(bad) && tid == 0) atomicOr(&st->flags, (unsigned)kStatusNonFinite);
-    if (tid == 0) atomicMax(&st->smax_bits, (unsigned long long)__double_as_longlong(vmax));
 }
 
 // ------------------------------------------------------------------------------------------

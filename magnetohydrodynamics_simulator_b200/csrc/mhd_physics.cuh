@@ -1,8 +1,8 @@
 // Per-cell and per-face FP64 physics of the reference solver, as device functions.
 //
-// Each function keeps the reference's arithmetic order (operand order of every sum and product),
-// so that the GPU path differs from the reference's CPU path only by FMA contraction and the
-// summation order of global reductions. References are to RikibabManos/Magnetohydrodynamics_Simulator.
+// The same expressions as the reference's, to rounding: quotients and roots by the approximations below, the fast
+// speed with one quotient under the root, the HLL cases through clamped wave speeds, and FMA contraction. Cells beyond
+// ordinary size keep the reference's own forms (ANY). References are to RikibabManos/Magnetohydrodynamics_Simulator.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -28,9 +28,9 @@ struct Flux {
 };
 
 // Reciprocal and square root as straight-line code: the hardware's approximation (relative error below
-// 2^-19; PTX rcp/rsqrt.approx.ftz.f64) and one third-order step (Householder 1970) for 1/a, one
-// Goldschmidt step and one residual correction (Markstein 1990) for sqrt(a). Largest error found against
-// the correctly rounded results, over 1.5e8 arguments of 2^-300 .. 2^300: 0.51 and 0.52 ulp. Their
+// 2^-19; PTX rcp/rsqrt.approx.ftz.f64) and one third-order step (Householder 1970) for 1/a and 1/sqrt(a), one
+// Goldschmidt step and one residual correction (Markstein 1990) for sqrt(a). Largest error found over 2^24 arguments of
+// 2^-300 .. 2^300 (a GPU test asserts these): 0.507 ulp for 1/a, 0.509 for sqrt(a), 1.00 for 1/sqrt(a), 1.94 for sqrt(X/r). Their
 // arguments are normal numbers, positive for the root (0, infinities and subnormals give NaN). The library's
 // division and root branch to a slow path, and each such branch ends a basic block: with the eight roots and
 // seven reciprocals of a cell's two faces inline, both faces' arithmetic interleaves.
