@@ -58,32 +58,38 @@ k_state_store(size_t n, CPlanes src, Planes dst) {
 
 namespace mhd_host {
 
-// Whether a kernel may use [p, p + bytes) as doubles: aligned memory of this device, inside one allocation. Anything
-// else (host, managed or another device's memory, ranges across allocations or too short) is left to the copy, which
-// accepts or refuses it.
+// A driver function, or null.
+inline void* driver_entry(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &found) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return found == cudaDriverEntryPointSuccess ? f : nullptr;
+}
+
+// Whether a kernel may use [p, p + bytes) as doubles: aligned memory of this device, inside one allocation, which is not
+// another context's (pool memory is no context's). Anything else (host, managed, another context's or device's memory,
+// ranges across allocations or too short) is left to the copy, which accepts or refuses it.
 inline bool plain_device_range(const void* p, size_t bytes, int device) {
     using GetAttributes = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
-    static const GetAttributes get = []() -> GetAttributes {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        return found == cudaDriverEntryPointSuccess ? (GetAttributes)f : nullptr;
-    }();
+    using GetCurrent = CUresult (*)(CUcontext*);
+    static const GetAttributes get = (GetAttributes)driver_entry("cuPointerGetAttributes");
+    static const GetCurrent current = (GetCurrent)driver_entry("cuCtxGetCurrent");
     const uintptr_t a = (uintptr_t)p;
-    if (!get || a % sizeof(double)) return false;
+    if (!get || !current || a % sizeof(double)) return false;
     unsigned int type = 0, managed = 1;
     int ordinal = -1;
     CUdeviceptr base = 0;
     size_t size = 0;
-    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+    CUcontext owner = nullptr, here = nullptr;
+    CUpointer_attribute what[6] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
                                    CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
-                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void* into[5] = {&type, &managed, &ordinal, &base, &size};
-    if (get(5, what, into, (CUdeviceptr)a) != CUDA_SUCCESS) return false;
-    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == device && base && a >= base &&
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_CONTEXT};
+    void* into[6] = {&type, &managed, &ordinal, &base, &size, &owner};
+    if (get(6, what, into, (CUdeviceptr)a) != CUDA_SUCCESS || current(&here) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == device && (!owner || owner == here) && base && a >= base &&
            a - base <= size && bytes <= size - (a - base);
 }
 
